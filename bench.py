@@ -50,13 +50,11 @@ sys.path.insert(0, ROOT)
 PKG = "springback-precomp_b200"
 METRIC = "Hex8 tangent+residual+assembly elem/s (FP64)"
 # DRAM bytes (read + write) per element of one evaluation's K1: ncu's
-# dram__bytes_read.sum + dram__bytes_write.sum summed over the phase kernels
-# of one evaluation of the same construction at 80,000 elements (200 x 200 x
-# 2): 16.57 GB (pre 4.48, return 5.41, log map 2.09, post 2.94, control
-# 0.48, condense 0.81, the single kernel's share 0.36); the traffic grows
-# with the elements, so an evaluation of ne elements moves about ne times
-# this.
-K1_DRAM_BYTES_PER_ELEMENT = 16.57e9 / 80000
+# dram__bytes_read.sum + dram__bytes_write.sum summed over its launches in one
+# evaluation of the same construction at 80,000 elements (200 x 200 x 2):
+# 1.71 GB (the tile kernel 0.63, the condensation 0.69, the single kernel's
+# share 0.38); the traffic grows with the elements.
+K1_DRAM_BYTES_PER_ELEMENT = 1.706e9 / 80000
 # The single kernel (--local-iteration single): 0.69 + 5.28 GB in one launch
 # at 80,000 elements.
 K1_SINGLE_DRAM_BYTES_PER_ELEMENT = (0.692594688e9 + 5.275133e9) / 80000
@@ -762,7 +760,7 @@ def run_cone(args, rank, world):
     if flops:
         achieved = flops * ne / (el_ms / 1e3) / 1e12
         roofline = {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                    "frac": achieved / fp64_peak, "traffic": None, "kernel": "K1 (phase kernels)",
+                    "frac": achieved / fp64_peak, "traffic": None, "kernel": "K1 (tile_kernel, condense_kernel)",
                     "kernel_ms": el_ms, "flops_per_element": flops,
                     "peak_source": "measured in this run: cuBLAS FP64 GEMM 8192^3 burst"}
     line = {"metric": METRIC + " with two-tool contact", "value": ne / (ms / 1e3), "unit": UNIT, "n_gpus": 1,
@@ -780,12 +778,12 @@ def run_cone(args, rank, world):
             "contact": {"begin_grid_ms": grid_ms, "begin_scan_ms": scan_ms, "candidates": grid_cand,
                         "active": [int(cev.tools[k][6]) for k in range(2)],
                         "slaves": [int(len(t["nodes"])) for t in prob.tools], "margin_m": margin},
-            # K1's phase kernels (26 rounds of 5, the condensation, the
-            # single kernel's list), K2b + finish, K2a; per tool 7 contact
+            # K1 (the tile kernel, the condensation, the single kernel's
+            # list), K2b + finish, K2a; per tool 7 contact
             # kernels (moved points, evaluate, the ordered compaction's 3,
             # scatter, resultants), the norms' two stages over both tools,
             # and the blocks' add.
-            "gpu_launches": args.steps * ((26 * 5 + 2) + 3 + 2 * 7 + 2 + 1), "clocks": clocks.summary(),
+            "gpu_launches": args.steps * (3 + 3 + 2 * 7 + 2 + 1), "clocks": clocks.summary(),
             "yielding_fraction": ev.yielding_points / (8.0 * ne),
             "setup_s": setup_s}
     print(json.dumps(line), flush=True)
@@ -992,7 +990,7 @@ def main():
     p.add_argument("--cpu-steps", type=int, default=5, help="timed steps of the in-run CPU baseline")
     p.add_argument("--epb", type=int, default=0, help="elements per block of the element kernel (0: default)")
     p.add_argument("--local-iteration", default="phases", choices=["phases", "single"],
-                   help="the local iteration as phase kernels over the mesh (default) or one kernel per element")
+                   help="the local iteration in tiles of elements (default) or one kernel per element")
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--no-e2e", action="store_true")
     p.add_argument("--cone-n", type=int, default=224)
@@ -1152,15 +1150,14 @@ def main():
                                       prob.mesh.gather(prob.u), committed, prob.alpha)
             flops_per_element = cnt / prob.mesh.num_elements
         el_ms = statistics.mean(elem_ms)
-        # Kernels of one step: K1 (the phase kernels: 26 rounds of 5 launches,
-        # the condensation, the single kernel for the elements it takes; or
-        # one launch), then the force gather and its finish (2), the value
-        # gather, and for the single kernel the schedule (count, CUB's scan,
-        # place).
+        # Kernels of one step: K1 (the tile kernel and the condensation per GiB
+        # of records, 614 doubles an element, and the single kernel for the
+        # elements these leave; or one launch), then the force gather and its
+        # finish (2), the value gather, and for the single kernel the schedule
+        # (count, CUB's scan, place).
         phases = args.element == "incompatible_modes" and args.local_iteration == "phases"
-        launches_per_step = (26 * 5 + 2 if phases else 1 + 3) + 3
-        k1_name = ("K1: the local iteration as phase kernels (wave_pre / wave_return / wave_log / wave_post / "
-                   "wave_control x 26 rounds, wave_condense, element_list)" if phases else
+        launches_per_step = (2 * -(-ne // ((1 << 30) // (614 * 8))) + 1 if phases else 1 + 3) + 3
+        k1_name = ("K1: the local iteration in tiles (tile_kernel, condense_kernel, element_list_kernel)" if phases else
                    "element_kernel (K1)" if args.element == "incompatible_modes" else "standard_kernel (K1s)")
         roofline = None
         if flops_per_element:

@@ -168,23 +168,25 @@ int sbk_system_element(const sbk_system* sys, int* element, int* averaged);
  * stiffness_gross act on the current one. */
 int sbk_system_set_values_buffer(sbk_system* sys, double* values_dev);
 
-/* Launch shape of the element kernel: elements per thread block (0: the
- * default, 16 for rules of up to 8 points - four warps - and 8 for larger
- * rules - eight warps; at most what 227 KB of shared memory and 256 threads
- * hold; the batch autotuner sets it). */
+/* Launch shape of the element kernel: elements per thread block. 0, the
+ * default: a tile of as many elements as the block has threads for their
+ * points (32 at 8 points, 12 at 20), fewer on a mesh too small to fill the
+ * GPU with full tiles; for the single kernel 16 for rules of up to 8 points
+ * - four warps - and 8 for larger rules - eight warps. At most what 227 KB of
+ * shared memory and 256 threads hold; the batch autotuner sets it. */
 int sbk_system_set_elements_per_block(sbk_system* sys, int elements_per_block);
 
 /* How the incompatible-mode Hex8's local iteration runs on the GPU (no
- * counterpart in the reference; no result depends on it - both give the
- * same outputs to the bit). SBK_LOCAL_PHASES (the default): phase kernels
- * over the whole mesh - each round a pass over the elements still
- * iterating, then their element-level step - with the elements that need a
- * line search, the shifted direction or Levenberg-Marquardt handed to the
- * single kernel; rules of up to 8 points (the others always take the single
- * kernel). SBK_LOCAL_SINGLE_KERNEL: one kernel runs each element from start
- * to finish. The phase kernels keep per-element records on the device
- * (about 6.7 KB per element, allocated by the system when it is made or its
- * element changes). sbk_set_local_iteration sets what sbk_element_batch
+ * counterpart in the reference; no decision depends on it, and the values
+ * only in their last bits). SBK_LOCAL_PHASES (the default): one kernel over
+ * tiles of elements, whose points and elements go through the phases of the
+ * iteration together on chip, then the condensation of all elements; the
+ * elements that need a line search, the shifted direction or
+ * Levenberg-Marquardt are handed to the single kernel. Every rule.
+ * SBK_LOCAL_SINGLE_KERNEL: one kernel runs each element from start to
+ * finish. The first keeps records of up to 1 GiB on the device (4.9 KB an
+ * element at 8 points, 10.9 KB at 20; allocated by the system when it is
+ * made or its element changes). sbk_set_local_iteration sets what sbk_element_batch
  * uses and what new systems start with. */
 #define SBK_LOCAL_PHASES 0
 #define SBK_LOCAL_SINGLE_KERNEL 1

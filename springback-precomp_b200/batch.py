@@ -78,10 +78,10 @@ class PartBatch:
     def autotune(self, u: torch.Tensor, candidates=(("phases", 0), ("phases", 8), ("single", 16), ("single", 8)),
                  repeats: int = 2, want_tangent: bool = True):
         """Time the element loop at each candidate mapping on this batch -
-        (local iteration, elements per block): the phase kernels (a thread
-        per point in the point kernels, an 8-lane group per element in the
-        others) or the single kernel (an 8-lane group per element, a point
-        per lane, start to finish), each at a block shape - with CUDA events
+        (local iteration, elements per block): the tile kernel (a thread per
+        point, 16 lanes per element in its control) or the single kernel (an
+        8-lane group per element, a point per lane, start to finish), each at
+        a block shape - with CUDA events
         on the system's stream after one warm-up; keep the fastest and
         return {candidate: ms}. No result depends on the choice. A bare
         integer candidate is an elements-per-block of the current mode."""

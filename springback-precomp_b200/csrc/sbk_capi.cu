@@ -330,6 +330,7 @@ int make_params(const sbk_material* mat, const sbk_rule* rule, int kinematics, P
     for (int i = 0; i < mat->num_backstresses; ++i) {
       p.termC[p.nterms] = mat->backstress_modulus[i];
       p.termG[p.nterms] = mat->backstress_recovery[i];
+      p.termGi[p.nterms] = p.termG[p.nterms] > 0.0 ? 1.0 / p.termG[p.nterms] : 0.0;
       ++p.nterms;
     }
     if (p.Hkin > 0.0) {
@@ -407,8 +408,8 @@ struct sbk_system {
   bool has_values = false;  // values hold the tangent of the last evaluate
   bool timing = false;
   int local_mode = SBK_LOCAL_PHASES;
-  void* wave_mem = nullptr;  // the phase kernels' records (one allocation)
-  sbk::WaveBuffers wave{};
+  void* tile_mem = nullptr;  // the tile kernel's scratch (one allocation)
+  sbk::TileScratch tile{};
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   double last_ms[3] = {0.0, 0.0, 0.0};
 
@@ -436,7 +437,7 @@ void free_system(sbk_system* s) {
                   s->tangent, s->energy_e, s->yield, s->iters, s->code, s->first_fail, s->outer,
                   s->inner, s->own_values, s->internal, s->scratch, s->scalars, s->missing, s->block_col,
                   s->block_value, s->block_ptr, s->block_src, s->node_ptr, s->node_src, s->product,
-                  s->order, s->sched, s->wave_mem};
+                  s->order, s->sched, s->tile_mem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (cudaEvent_t e : s->ev)
@@ -446,38 +447,36 @@ void free_system(sbk_system* s) {
 
 std::atomic<int> g_local_mode{SBK_LOCAL_PHASES};
 
-// The phase kernels' records of a system whose element takes them
-// (allocated once, outside any stream capture).
-int ensure_wave(sbk_system* s) {
-  if (s->wave_mem || !sbk::wave_applies(s->p)) return SBK_OK;
-  const size_t bytes = sbk::wave_buffer_bytes(s->ne);
-  cudaError_t e = cudaMalloc(&s->wave_mem, bytes);
+// The tile kernel's scratch of a system whose element takes it (allocated
+// once, outside any stream capture).
+int ensure_tile(sbk_system* s) {
+  if (s->tile_mem || !sbk::tile_applies(s->p)) return SBK_OK;
+  cudaError_t e = cudaMalloc(&s->tile_mem, sbk::tile_scratch_bytes(s->ne, s->p.nq));
   if (e != cudaSuccess) {
-    s->wave_mem = nullptr;
-    return fail(SBK_ERR_CUDA, std::string("cudaMalloc (local-iteration records): ") + cudaGetErrorString(e));
+    s->tile_mem = nullptr;
+    return fail(SBK_ERR_CUDA, std::string("cudaMalloc (tile scratch): ") + cudaGetErrorString(e));
   }
-  sbk::wave_buffers_carve(s->wave_mem, s->ne, s->wave);
+  sbk::tile_scratch_carve(s->tile_mem, s->ne, s->p.nq, s->tile);
   return SBK_OK;
 }
 
-// Whether K1 of the system runs as the phase kernels.
-bool uses_phases(const sbk_system* sys) {
-  return sys->local_mode == SBK_LOCAL_PHASES && sys->wave_mem && sbk::wave_applies(sys->p);
+// Whether K1 of the system runs as the tile kernel.
+bool uses_tiles(const sbk_system* sys) {
+  return sys->local_mode == SBK_LOCAL_PHASES && sys->tile_mem && sbk::tile_applies(sys->p);
 }
 
 // Whether the element schedule runs after an evaluation: for the single
-// kernel only. The phase kernels take the elements in mesh order (on the
-// 1M-element microbenchmark the schedule's order was 0.5 % slower there:
-// every phase is a short body of code that all warps share anyway).
-bool schedules(const sbk_system* sys) { return sys->schedule && !uses_phases(sys); }
+// kernel only. The tile kernel takes the elements in mesh order: its stages
+// keep the warps of a block on the same code whatever their elements do.
+bool schedules(const sbk_system* sys) { return sys->schedule && !uses_tiles(sys); }
 
-// K1 of a system: the phase kernels where they apply, else the single kernel.
+// K1 of a system: the tile kernel where it applies, else the single kernel.
 int system_elements(sbk_system* sys, const double* u_dev, int want_tangent, cudaStream_t st) {
   const int32_t* order = sys->schedule && sys->order_valid ? sys->order : nullptr;
-  if (uses_phases(sys))
-    return sbk::launch_elements_wave(sys->p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c,
+  if (uses_tiles(sys))
+    return sbk::launch_elements_tile(sys->p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c,
                                      want_tangent, sys->force, sys->tangent, sys->energy_e, sys->trial, sys->alpha_t,
-                                     sys->yield, sys->iters, sys->code, sys->first_fail, false, nullptr, sys->wave,
+                                     sys->yield, sys->iters, sys->code, sys->first_fail, false, sys->tile,
                                      sys->elements_per_block, st);
   return sbk::launch_elements(sys->p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c,
                               want_tangent, sys->force, sys->tangent, sys->energy_e, sys->trial, sys->alpha_t,
@@ -545,15 +544,15 @@ int sbk_element_batch(const sbk_material* material, const sbk_rule* rule, int ki
     return fail(SBK_ERR_ARGUMENT, "null device buffer");
   if (ne * p.nq > 0x7fffffffLL) return fail(SBK_ERR_UNSUPPORTED, "too many points for one batch");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (g_local_mode.load() == SBK_LOCAL_PHASES && sbk::wave_applies(p)) {
-    // The phase kernels' records, stream-ordered on the caller's stream.
+  if (g_local_mode.load() == SBK_LOCAL_PHASES && sbk::tile_applies(p)) {
+    // The tile kernel's scratch, stream-ordered on the caller's stream.
     void* mem = nullptr;
-    SBK_CUDA(cudaMallocAsync(&mem, sbk::wave_buffer_bytes(ne), s));
-    sbk::WaveBuffers w;
-    sbk::wave_buffers_carve(mem, ne, w);
-    rc = sbk::launch_elements_wave(p, ne, x_dev, nullptr, u_dev, state_dev, alpha_dev, tangent_dev != nullptr,
+    SBK_CUDA(cudaMallocAsync(&mem, sbk::tile_scratch_bytes(ne, p.nq), s));
+    sbk::TileScratch w;
+    sbk::tile_scratch_carve(mem, ne, p.nq, w);
+    rc = sbk::launch_elements_tile(p, ne, x_dev, nullptr, u_dev, state_dev, alpha_dev, tangent_dev != nullptr,
                                    force_dev, tangent_dev, energy_dev, trial_dev, alpha_out_dev, yield_dev,
-                                   iterations_dev, code_dev, nullptr, true, nullptr, w, 0, s);
+                                   iterations_dev, code_dev, nullptr, true, w, 0, s);
     cudaError_t e = cudaFreeAsync(mem, s);
     if (rc) return fail(SBK_ERR_CUDA, std::string("element kernels: ") + cudaGetErrorString((cudaError_t)rc));
     if (e != cudaSuccess) return fail(SBK_ERR_CUDA, std::string("cudaFreeAsync: ") + cudaGetErrorString(e));
@@ -639,7 +638,7 @@ int sbk_system_create(const sbk_mesh* mesh, const sbk_material* material, const 
   TRY(dalloc(&s->scalars, 4));
   TRY(dalloc(&s->missing, 1));
   s->local_mode = g_local_mode.load();
-  TRY(ensure_wave(s));
+  TRY(ensure_tile(s));
 #undef TRY
   // Virgin points and zero modes (initialise_history).
   cudaMemset(s->committed, 0, state_size * sizeof(double));
@@ -691,11 +690,11 @@ int sbk_system_set_element(sbk_system* sys, int element, int mean_dilatation) {
                         ? 1
                         : 0;
   sys->order_valid = false;
-  if (!sbk::wave_applies(sys->p) && sys->wave_mem) {
-    cudaFree(sys->wave_mem);
-    sys->wave_mem = nullptr;
+  if (!sbk::tile_applies(sys->p) && sys->tile_mem) {
+    cudaFree(sys->tile_mem);
+    sys->tile_mem = nullptr;
   }
-  return sys->local_mode == SBK_LOCAL_PHASES ? ensure_wave(sys) : SBK_OK;
+  return sys->local_mode == SBK_LOCAL_PHASES ? ensure_tile(sys) : SBK_OK;
 }
 
 int sbk_system_set_frozen(sbk_system* sys, int frozen) {
@@ -731,7 +730,7 @@ int sbk_system_set_local_iteration(sbk_system* sys, int mode) {
   if (!sys) return fail(SBK_ERR_ARGUMENT, "null system");
   if (mode != SBK_LOCAL_PHASES && mode != SBK_LOCAL_SINGLE_KERNEL) return fail(SBK_ERR_ARGUMENT, "unknown mode");
   sys->local_mode = mode;
-  return mode == SBK_LOCAL_PHASES ? ensure_wave(sys) : SBK_OK;
+  return mode == SBK_LOCAL_PHASES ? ensure_tile(sys) : SBK_OK;
 }
 
 int sbk_system_set_values_buffer(sbk_system* sys, double* values_dev) {

@@ -23,20 +23,12 @@
 #include <stdint.h>
 
 #include "sbk_element.h"
+#include "sbk_element_math.cuh"
 #include "sbk_material.cuh"
-#include "sbk_wave.h"
+#include "sbk_tile.h"
 
 namespace sbk {
 namespace {
-
-constexpr int kMaxLocal = 25;
-constexpr double kFullStepReduction = 1.0 - 1.0e-4;
-constexpr int kMaxLineSearch = 8;
-constexpr double kLineSearchRatio = 0.5;
-constexpr double kLocalShift = 1.0e-3;
-constexpr double kLocalMarquardt = 1.0e-6;
-constexpr double kLocalTolerance = 1.0e-8;
-constexpr double kLocalRoundOff = 1.0e-13;
 
 constexpr int kSlot = 54;  // per point: D 36 | S 6 | F 9 | w | energy | floor factor
 constexpr int kSlotS = 36, kSlotF = 42, kSlotW = 51, kSlotE = 52, kSlotFl = 53;
@@ -80,46 +72,6 @@ __device__ __forceinline__ void shape_grad(int a, double xi, double eta, double 
   dn[0] = 0.125 * kCorner[a][0] * fy * fz;
   dn[1] = 0.125 * kCorner[a][1] * fx * fz;
   dn[2] = 0.125 * kCorner[a][2] * fx * fy;
-}
-
-__device__ __forceinline__ double det3(const double m[9]) {
-  return m[0] * (m[4] * m[8] - m[7] * m[5]) - m[3] * (m[1] * m[8] - m[7] * m[2]) +
-         m[6] * (m[1] * m[5] - m[4] * m[2]);
-}
-__device__ __forceinline__ void inv3(const double m[9], double out[9]) {
-  out[0] = m[4] * m[8] - m[5] * m[7];
-  out[3] = m[5] * m[6] - m[3] * m[8];
-  out[6] = m[3] * m[7] - m[4] * m[6];
-  const double det = m[0] * out[0] + m[1] * out[3] + m[2] * out[6];
-  const double inv = 1.0 / det;
-  out[1] = m[2] * m[7] - m[1] * m[8];
-  out[4] = m[0] * m[8] - m[2] * m[6];
-  out[7] = m[1] * m[6] - m[0] * m[7];
-  out[2] = m[1] * m[5] - m[2] * m[4];
-  out[5] = m[2] * m[3] - m[0] * m[5];
-  out[8] = m[0] * m[4] - m[1] * m[3];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) out[i] *= inv;
-}
-
-// Reduce-scatter of G values over the G lanes of a group: lane l returns the
-// group sum of v[l]. Fixed pairing, so the result is deterministic.
-template <int G>
-__device__ __forceinline__ double reduce_scatter(double (&v)[G], int lane, unsigned mask) {
-  double cur[G];
-#pragma unroll
-  for (int i = 0; i < G; ++i) cur[i] = v[i];
-#pragma unroll
-  for (int half = G / 2; half >= 1; half >>= 1) {
-    const bool upper = (lane & half) != 0;
-#pragma unroll
-    for (int j = 0; j < half; ++j) {
-      const double send = upper ? cur[j] : cur[half + j];
-      const double keep = upper ? cur[half + j] : cur[j];
-      cur[j] = keep + __shfl_xor_sync(mask, send, half, G);
-    }
-  }
-  return cur[0];
 }
 
 // Voigt index of the tensor pair (i, j).
@@ -191,8 +143,7 @@ __device__ __forceinline__ void vtensor(const double* slot, const double g[3], b
 }
 
 // The per-element context of a group: S is the shared-memory record of one
-// element, which differs between the single element kernel and the phase
-// kernels (each holds only the fields its stage reads).
+// element.
 template <int G, class Rec = ElemShared<G>>
 struct Ctx {
   const Params* p;
@@ -1428,7 +1379,7 @@ __global__ void __launch_bounds__(256) element_kernel(const __grid_constant__ Pa
 }
 
 // The single kernel over a device-counted list of elements (grid-stride):
-// the phase kernels hand it the elements that leave their common road.
+// the tile kernel hands it the elements that leave its common road.
 template <int G>
 __global__ void __launch_bounds__(256) element_list_kernel(const __grid_constant__ Params p, int64_t ne, bool batch,
                                                            const double* __restrict__ coords,
@@ -1457,593 +1408,6 @@ __global__ void __launch_bounds__(256) element_list_kernel(const __grid_constant
     __syncwarp(mask);
     element_body<G>(p, ne, batch, (int64_t)list[i], sh, lane, mask, coords, conn, u, state, alpha_n, want_tangent,
                     force, tangent, energy, trial, alpha_out, yield, iterations, code, first_failure);
-  }
-}
-
-// ---- the local iteration as phase kernels over the whole mesh ------------------
-//
-// The same algorithm as element_kernel, split at its passes. Every element
-// of the mesh runs its local iteration in lockstep rounds; a round is two
-// launches over the elements still iterating:
-//
-//   wave_pass_kernel     one pass at each element's trial modes (the first
-//                        round: the geometry, then the pass at alpha_n);
-//   wave_control_kernel  the element-level step that follows a pass: the
-//                        full-pivoting LU of K_aa and the convergence test,
-//                        Newton's direction and the Cholesky test of the
-//                        symmetric part, the acceptance of a full step.
-//
-// Most elements take only that road - every trial a full Newton step that
-// the residual test accepts. An element that needs anything else (a step
-// the test rejects, a trial pass that fails, an indefinite K_aa, hence the
-// line searches, the shifted direction or Levenberg-Marquardt) is handed to
-// element_kernel, which runs it again from the start; an element that
-// converges goes to wave_condense_kernel, the condensation. Elements
-// continuing to the next round are compacted into the next round's list.
-// The passes, the factorisations, the tests and the condensation are the
-// single kernel's own functions on the same values, so every element's
-// outputs are bit-identical to element_kernel's (tested), and the rounds
-// end by construction: the first pass plus at most kMaxLocal Newton steps.
-//
-// Why: the single kernel runs set-up, passes, 9 x 9 algebra and
-// condensation back to back in one body of about 470 KB of code with 9.8 KB
-// of shared memory per element - one 4-warp block per SM, its warps at
-// different places in the code. Each phase kernel is a fraction of that
-// code, its record a fraction of that memory, and the warps of a launch all
-// run the same phase.
-
-constexpr int kWaveRounds = kMaxLocal + 1;
-constexpr int kKcStride = 88;  // K_aa as the reduce-scatter leaves it (81 used)
-
-template <int G>
-struct __align__(16) PassShared {
-  double X[24];
-  double U[24];
-  double jinv0[9];
-  double geo[G][12];
-  double slot[G][kSlot];
-  double kc[kKcStride];
-  double r[33];
-  double scale[9];
-  double flo[9];
-  double energy;
-};
-
-// The first pass kernel's record: the staged element and its geometry.
-template <int G>
-struct __align__(16) PreShared {
-  double X[24];
-  double U[24];
-  double jinv0[9];
-  double geo[G][12];
-};
-
-// Minimum resident blocks per SM (128 threads each) the compiler is told
-// to fit, which bounds the registers of a thread: 2 allows 255, 3 170, 4
-// 128. Measured on the 1M-element microbenchmark: these kernels lose 15-65 %
-// at 3 or 4 (their spills grow), the logarithmic map 33 % at 3; the return
-// kernel (sbk_return.cu) is best at 4.
-#ifndef SBK_MINB_PRE
-#define SBK_MINB_PRE 2
-#endif
-#ifndef SBK_MINB_POST
-#define SBK_MINB_POST 2
-#endif
-#ifndef SBK_MINB_LOG
-#define SBK_MINB_LOG 2
-#endif
-#ifndef SBK_MINB_CONDENSE
-#define SBK_MINB_CONDENSE 2
-#endif
-
-// The control kernel's record: K_aa (then, once the LU has copied it, its
-// symmetric part in place for the Cholesky test), the LU, the pass's sums.
-// 1.9 KB per element, so that six 4-warp blocks fit an SM (the kernel's
-// registers allow six).
-template <int G>
-struct __align__(16) ControlShared {
-  double kc[81];
-  double lu[81];
-  double r[33];
-  double scale[9];
-  double flo[9];
-  double alpha[9];
-  double dir[9];
-  double maxpivot;
-  int rowp[9], colp[9];
-};
-
-template <int G>
-struct __align__(16) CondenseShared {
-  double jinv0[9];
-  double geo[G][12];
-  double slot[G][kSlot];
-  double kc[216];
-  double r[33];
-  double lu[81];
-  int rowp[9], colp[9];
-  double energy;
-};
-
-__device__ __forceinline__ double modes_norm(const double* r) {
-  double v = 0.0;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) v += r[24 + i] * r[24 + i];
-  return sqrt(v);
-}
-__device__ __forceinline__ double modes_inf(const double* r) {
-  double v = fabs(r[24]);
-#pragma unroll
-  for (int i = 1; i < 9; ++i) v = fmax(v, fabs(r[24 + i]));
-  return v;
-}
-__device__ __forceinline__ double abs_max9(const double* v) {
-  double m = fabs(v[0]);
-#pragma unroll
-  for (int i = 1; i < 9; ++i) m = fmax(m, fabs(v[i]));
-  return m;
-}
-
-// Warp-aggregated append of element e (by lane 0 of its group) to a list.
-__device__ __forceinline__ void append(int32_t* list, int32_t* count, int64_t e) {
-  const int pos = atomicAdd(count, 1);
-  list[pos] = (int32_t)e;
-}
-
-// Pass, first kernel: per point the kinematics at the trial modes and the
-// log strain; the response of every point the return takes elastically,
-// here; the points that will yield listed for wave_return_kernel. The first
-// round also stages the element and runs set_up.
-template <int G, bool GENERAL>
-__global__ void __launch_bounds__(128, SBK_MINB_PRE) wave_pre_kernel(const __grid_constant__ Params p, int64_t ne, int first,
-                                                       const int32_t* __restrict__ list,
-                                                       const int32_t* __restrict__ count, bool batch,
-                                                       const double* __restrict__ coords,
-                                                       const int32_t* __restrict__ conn,
-                                                       const double* __restrict__ u, const double* __restrict__ state,
-                                                       const double* __restrict__ alpha_n,
-                                                       double* __restrict__ trial, uint8_t* __restrict__ yield,
-                                                       int32_t* __restrict__ plastic,
-                                                       int32_t* __restrict__ plastic_count,
-                                                       const __grid_constant__ WaveBuffers w) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int epb = blockDim.x / G;
-  const int slot_in_block = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  PreShared<G>* sh = reinterpret_cast<PreShared<G>*>(smem_raw) + slot_in_block;
-  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
-  const int64_t n = count ? (int64_t)*count : ne;
-  const int nq = p.nq;
-  PreShared<G>& s = *sh;
-  for (int64_t i = (int64_t)blockIdx.x * epb + slot_in_block; i < n; i += (int64_t)gridDim.x * epb) {
-    const int64_t e = list ? (int64_t)list[i] : i;
-    double hu_lane[9];
-    double* warm = w.warm + (e * 8 + lane) * 8;
-    Ctx<G, PreShared<G>> c{&p, sh, lane, mask, e, ne * nq, state, trial, yield, hu_lane, warm};
-    __syncwarp(mask);
-    int status = 0;
-    double at[9];
-    if (first) {
-      // The single kernel's start: staging (a node out of range fails the
-      // element), alpha_n, set_up.
-      int bad_node = 0;
-      if (lane < 8) {
-        if (batch) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            s.X[3 * lane + k] = coords[e * 24 + 3 * lane + k];
-            s.U[3 * lane + k] = u[e * 24 + 3 * lane + k];
-          }
-        } else {
-          const int64_t node = conn[e * 8 + lane];
-          if (p.num_nodes > 0 && (node < 0 || node >= p.num_nodes)) {
-            bad_node = 1;
-          } else {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              s.X[3 * lane + k] = coords[node * 3 + k];
-              s.U[3 * lane + k] = u[node * 3 + k];
-            }
-          }
-        }
-      }
-      if (__any_sync(mask, bad_node)) {
-        status = SBK_EL_BAD_NODE;
-      } else {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) at[k] = alpha_n ? alpha_n[e * 9 + k] : 0.0;
-        for (int k = lane; k < 9; k += G) w.alpha[e * 9 + k] = at[k];
-        if (lane < 8)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) warm[k] = 0.0;  // no closest point yet (warm[7] == 0)
-        c.sync();
-        status = set_up<G>(c);
-        if (!status) {
-          if (lane < nq) {
-#pragma unroll
-            for (int f = 0; f < 12; ++f) w.geo[(e * 12 + f) * G + lane] = s.geo[lane][f];
-#pragma unroll
-            for (int f = 0; f < 9; ++f) w.hu[(e * 9 + f) * G + lane] = hu_lane[f];
-          }
-          for (int k = lane; k < 9; k += G) w.jinv0[e * 9 + k] = s.jinv0[k];
-        }
-      }
-    } else {
-      // A trial at alpha + 1 dir (Local::try_at with t = 1).
-#pragma unroll
-      for (int k = 0; k < 9; ++k) at[k] = w.alpha[e * 9 + k] + 1.0 * w.dir[e * 9 + k];
-      if (lane < nq) {
-#pragma unroll
-        for (int f = 0; f < 12; ++f) s.geo[lane][f] = w.geo[(e * 12 + f) * G + lane];
-#pragma unroll
-        for (int f = 0; f < 9; ++f) hu_lane[f] = w.hu[(e * 9 + f) * G + lane];
-      }
-      for (int k = lane; k < 9; k += G) s.jinv0[k] = w.jinv0[e * 9 + k];
-      c.sync();
-    }
-    // An element that failed before its points: every point's record says
-    // so (stage 0 sorts before the points' own failures).
-    int fail = status ? 1 : 0, code = status;
-    bool deferred = false;
-    const int q = lane;
-    if (!status && q < nq) {
-      double gt[9], F[9], hmax = 0.0, strain[6];
-      LogKin L;
-      code = point_kinematics(c, q, at, gt, F, hmax, strain, L);
-      if (code) fail = (1 << 8) | q;
-      if (!fail) {
-        PointState st{state + e * nq + q, trial + e * nq + q, ne * nq};
-        Response r;
-        if (GENERAL) {
-          // The return's own trial test: its elastic branch outside the
-          // loading window here; the rest (the whole return again) in
-          // wave_return_kernel.
-          GTrial T;
-          general_trial(p, strain, st, T);
-          if (!isfinite(T.f_trial)) {
-            code = kFailReturn;
-          } else if (general_is_elastic(p, T) && !general_loading_window(p, T)) {
-            code = general_elastic<false>(p, T, st, r);
-          } else {
-            deferred = true;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) *pw_at(w, e, kPwStrain + k, q) = strain[k];
-          }
-        } else {
-          code = radial_return(p, strain, st, r);
-        }
-        if (code) fail = (2 << 8) | q;
-        else if (!deferred) store_response(w, e, q, r);
-      }
-#pragma unroll
-      for (int k = 0; k < 9; ++k) *pw_at(w, e, kPwF + k, q) = F[k];
-      *pw_at(w, e, kPwHmax, q) = hmax;
-#pragma unroll
-      for (int k = 0; k < 9; ++k) *pw_at(w, e, kPwL + k, q) = L.q[k];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) *pw_at(w, e, kPwL + 9 + k, q) = L.mu[k];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) *pw_at(w, e, kPwL + 12 + k, q) = L.first[k];
-    }
-    if (q < 8) {
-      w.pfail[e * 8 + q] = fail;
-      w.pcodes[e * 8 + q] = code;
-    }
-    // The group's deferred points, appended together.
-    const unsigned ballot = __ballot_sync(mask, deferred);
-    int base = 0;
-    if (ballot) {
-      const unsigned mine = ballot >> ((threadIdx.x % 32) / G * G);
-      if (lane == 0) base = atomicAdd(plastic_count, __popc(mine));
-      base = __shfl_sync(mask, base, 0, G);
-      if (deferred) plastic[base + __popc(mine & ((1u << lane) - 1u))] = (int32_t)(e * 8 + q);
-    }
-  }
-}
-
-// Pass, second kernel: the general return of every listed point, in
-// sbk_return.cu (launch_wave_returns).
-
-// Pass, third kernel (logarithmic kinematics): the logarithmic map of every
-// evaluated point's response (log_transform: S = P^T T, material = P^T C P
-// + T : L), a thread per point, in place in the point's record. On its own
-// its working set fits the registers of a thread; inside the sums kernel it
-// spilled.
-__global__ void __launch_bounds__(128, SBK_MINB_LOG) wave_log_kernel(int64_t ne, int nq, const int32_t* __restrict__ list,
-                                                          const int32_t* __restrict__ count,
-                                                          const __grid_constant__ WaveBuffers w) {
-  const int64_t n = (count ? (int64_t)*count : ne) * 8;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int q = (int)(i & 7);
-    if (q >= nq) continue;
-    const int64_t e = list ? (int64_t)list[i >> 3] : (i >> 3);
-    if (w.pfail[e * 8 + q]) continue;
-    LogKin L;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) L.q[k] = *pw_at(w, e, kPwL + k, q);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) L.mu[k] = *pw_at(w, e, kPwL + 9 + k, q);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) L.first[k] = *pw_at(w, e, kPwL + 12 + k, q);
-    double t[6], S[6], M[36];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) t[k] = *pw_at(w, e, kPwStress + k, q);
-#pragma unroll
-    for (int k = 0; k < 36; ++k) M[k] = *pw_at(w, e, kPwC + k, q);
-    log_transform(L, t, S, M);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) *pw_at(w, e, kPwStress + k, q) = S[k];
-#pragma unroll
-    for (int k = 0; k < 36; ++k) *pw_at(w, e, kPwC + k, q) = M[k];
-  }
-}
-
-// Pass, fourth kernel: per point the yield flag and the slot; per element
-// the first failure, K_aa and the sums (pass_sums) into the element's
-// record.
-template <int G>
-__global__ void __launch_bounds__(128, SBK_MINB_POST) wave_post_kernel(const __grid_constant__ Params p, int64_t ne,
-                                                        const int32_t* __restrict__ list,
-                                                        const int32_t* __restrict__ count,
-                                                        uint8_t* __restrict__ yield,
-                                                        const __grid_constant__ WaveBuffers w) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int epb = blockDim.x / G;
-  const int slot_in_block = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  PassShared<G>* sh = reinterpret_cast<PassShared<G>*>(smem_raw) + slot_in_block;
-  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
-  const int64_t n = count ? (int64_t)*count : ne;
-  const int nq = p.nq;
-  PassShared<G>& s = *sh;
-  for (int64_t i = (int64_t)blockIdx.x * epb + slot_in_block; i < n; i += (int64_t)gridDim.x * epb) {
-    const int64_t e = list ? (int64_t)list[i] : i;
-    Ctx<G, PassShared<G>> c{&p, sh, lane, mask, e, ne * nq, nullptr, nullptr, yield, nullptr, nullptr};
-    __syncwarp(mask);
-    const int q = lane;
-    const bool active = q < nq;
-    int fail = 0, code = 0;
-    if (q < 8) {
-      fail = w.pfail[e * 8 + q];
-      code = w.pcodes[e * 8 + q];
-    }
-    // A failure before the points (stage 0): the whole element.
-    const int early = __shfl_sync(mask, fail == 1 ? code : 0, 0, G);
-    if (early) {
-      if (lane == 0) w.pcode[e] = early;
-      continue;
-    }
-    if (active) {
-#pragma unroll
-      for (int f = 0; f < 12; ++f) s.geo[q][f] = w.geo[(e * 12 + f) * G + q];
-    }
-    for (int k = lane; k < 9; k += G) s.jinv0[k] = w.jinv0[e * 9 + k];
-    c.sync();
-    double gt[9], F[9], M[36], S[6], w_q = 0.0;
-    if (active) {
-      w_q = s.geo[q][9];
-      mode_grads(c, q, gt);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) F[k] = *pw_at(w, e, kPwF + k, q);
-      if (!fail) {
-        // The response in the element's strain measure (wave_log_kernel
-        // applied the logarithmic map).
-        Response r;
-        LogKin L;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) r.stress[k] = *pw_at(w, e, kPwStress + k, q);
-#pragma unroll
-        for (int k = 0; k < 36; ++k) r.C[k] = *pw_at(w, e, kPwC + k, q);
-        r.energy = *pw_at(w, e, kPwEnergy, q);
-        r.yielding = *pw_at(w, e, kPwYield, q) != 0.0;
-        const double hmax = *pw_at(w, e, kPwHmax, q);
-        point_slot<G, PassShared<G>, true>(c, q, r, L, F, w_q, hmax, M, S);
-      }
-    }
-    // The sums read the point's M, S and F back from its slot in shared
-    // memory, so that they need not stay in registers.
-    const double* sl = s.slot[q < nq ? q : 0];
-    const int status = pass_sums<G, PassShared<G>, false>(c, active, fail, code, gt, sl + kSlotF, sl, sl + kSlotS, w_q);
-    if (lane == 0) w.pcode[e] = status;
-    if (!status) {
-      for (int k = lane; k < 81; k += G) w.kc[e * kKcStride + k] = s.kc[k];
-      for (int k = lane; k < 9; k += G) {
-        w.r[e * 33 + 24 + k] = s.r[24 + k];
-        w.sf[e * 19 + k] = s.scale[k];
-        w.sf[e * 19 + 9 + k] = s.flo[k];
-      }
-      if (active) {
-#pragma unroll 6
-        for (int f = 0; f < kSlot; ++f) w.slot[(e * kSlot + f) * G + q] = s.slot[q][f];
-      }
-    }
-  }
-}
-
-// A failed element: its status and the lowest failing element, as the
-// single kernel reports them.
-__device__ __forceinline__ void wave_fail(int32_t* code, int32_t* first_failure, int64_t e, int status) {
-  code[e] = status;
-  if (first_failure) atomicMin(first_failure, (int32_t)e);
-}
-
-template <int G>
-__global__ void __launch_bounds__(128) wave_control_kernel(const __grid_constant__ Params p, int64_t ne, int first,
-                                                           const int32_t* __restrict__ list,
-                                                           const int32_t* __restrict__ count,
-                                                           const __grid_constant__ WaveBuffers w,
-                                                           int32_t* __restrict__ next, int32_t* __restrict__ next_count,
-                                                           int32_t* __restrict__ code,
-                                                           int32_t* __restrict__ first_failure) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int epb = blockDim.x / G;
-  const int slot_in_block = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  ControlShared<G>* sh = reinterpret_cast<ControlShared<G>*>(smem_raw) + slot_in_block;
-  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
-  const int64_t n = count ? (int64_t)*count : ne;
-  ControlShared<G>& s = *sh;
-  int32_t* done_list = w.done;
-  int32_t* done_count = w.counts + kWaveRounds + 1;
-  int32_t* fallback_list = w.fallback;
-  int32_t* fallback_count = w.counts + kWaveRounds + 2;
-  for (int64_t i = (int64_t)blockIdx.x * epb + slot_in_block; i < n; i += (int64_t)gridDim.x * epb) {
-    const int64_t e = list ? (int64_t)list[i] : i;
-    Ctx<G, ControlShared<G>> c{&p, sh, lane, mask, e, 0, nullptr, nullptr, nullptr, nullptr, nullptr};
-    __syncwarp(mask);
-    const int pc = w.pcode[e];
-    if (pc) {
-      // A failed first pass fails the element (Local::run); a failed trial
-      // is the line search's business.
-      if (lane == 0) {
-        if (first) wave_fail(code, first_failure, e, pc);
-        else append(fallback_list, fallback_count, e);
-      }
-      continue;
-    }
-    for (int k = lane; k < 81; k += G) s.kc[k] = w.kc[e * kKcStride + k];
-    for (int k = lane; k < 33; k += G) s.r[k] = w.r[e * 33 + k];
-    for (int k = lane; k < 9; k += G) {
-      s.scale[k] = w.sf[e * 19 + k];
-      s.flo[k] = w.sf[e * 19 + 9 + k];
-      s.alpha[k] = w.alpha[e * 9 + k];
-      s.dir[k] = w.dir[e * 9 + k];
-    }
-    int iterations = first ? 0 : w.iters[e];
-    double residual = first ? 0.0 : w.res[e];
-    c.sync();
-    if (first) {
-      residual = modes_norm(s.r);
-    } else {
-      // line_search's full step (IncompatibleModes.cpp:398-410): accepted
-      // when it reduces the residual enough or meets the tolerance.
-      const double full = modes_norm(s.r);
-      if (full <= kFullStepReduction * residual ||
-          modes_inf(s.r) <= kLocalTolerance * abs_max9(s.scale) + kLocalRoundOff * abs_max9(s.flo)) {
-        c.sync();
-        if (lane == 0)
-#pragma unroll
-          for (int k = 0; k < 9; ++k) s.alpha[k] += 1.0 * s.dir[k];
-        c.sync();
-        residual = full;
-      } else {
-        if (lane == 0) append(fallback_list, fallback_count, e);
-        continue;
-      }
-    }
-    // The head of solve_and_condense's loop (IncompatibleModes.cpp:353-397).
-    const double largest = modes_inf(s.r);
-    const double scale = abs_max9(s.scale);
-    const double floor_ = kLocalRoundOff * abs_max9(s.flo);
-    const bool invertible = fullpiv_lu9_rows_inline<G>(c, s.kc, s.lu, s.rowp, s.colp, &s.maxpivot);
-    c.sync();
-    if (!invertible) {
-      if (lane == 0) wave_fail(code, first_failure, e, SBK_EL_LOCAL_SINGULAR);
-      continue;
-    }
-    if (largest <= kLocalTolerance * scale + floor_ || largest == 0.0) {
-      // Converged: the factors of this K_aa for the condensation.
-      for (int k = lane; k < 81; k += G) w.kc[e * kKcStride + k] = s.lu[k];
-      for (int k = lane; k < 9; k += G) {
-        w.piv[e * 18 + k] = s.rowp[k];
-        w.piv[e * 18 + 9 + k] = s.colp[k];
-        w.alpha[e * 9 + k] = s.alpha[k];
-      }
-      if (lane == 0) {
-        w.iters[e] = iterations;
-        append(done_list, done_count, e);
-      }
-      continue;
-    }
-    if (iterations == kMaxLocal || !isfinite(largest)) {
-      if (lane == 0) wave_fail(code, first_failure, e, SBK_EL_LOCAL_NO_CONVERGE);
-      continue;
-    }
-    ++iterations;
-    // The symmetric part (K + K^T) / 2 in place: each lane owns the pairs
-    // (a, b), a <= b, it writes, and reads nothing another lane writes.
-    for (int idx = lane; idx < 45; idx += G) {
-      int a = 0, rest = idx;
-      while (rest >= 9 - a) {
-        rest -= 9 - a;
-        ++a;
-      }
-      const int b = a + rest;
-      const double v = 0.5 * (s.kc[a * 9 + b] + s.kc[b * 9 + a]);
-      s.kc[a * 9 + b] = v;
-      s.kc[b * 9 + a] = v;
-    }
-    c.sync();
-    if (lane == 0) {
-      double nw[9];
-      fullpiv_solve9_inline(s.lu, s.rowp, s.colp, s.r + 24, nw);
-      for (int k = 0; k < 9; ++k) s.dir[k] = -nw[k];
-    }
-    const bool positive = llt9_rows_inline<G>(c, s.kc);
-    c.sync();
-    if (!positive) {
-      if (lane == 0) append(fallback_list, fallback_count, e);
-      continue;
-    }
-    for (int k = lane; k < 9; k += G) {
-      w.alpha[e * 9 + k] = s.alpha[k];
-      w.dir[e * 9 + k] = s.dir[k];
-    }
-    if (lane == 0) {
-      w.iters[e] = iterations;
-      w.res[e] = residual;
-      append(next, next_count, e);
-    }
-  }
-}
-
-template <int G>
-__global__ void __launch_bounds__(128, SBK_MINB_CONDENSE) wave_condense_kernel(const __grid_constant__ Params p, int64_t ne,
-                                                            const __grid_constant__ WaveBuffers w, int want_tangent,
-                                                            double* __restrict__ force, double* __restrict__ tangent,
-                                                            double* __restrict__ energy,
-                                                            double* __restrict__ alpha_out,
-                                                            int32_t* __restrict__ iterations,
-                                                            int32_t* __restrict__ code) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int epb = blockDim.x / G;
-  const int slot_in_block = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  CondenseShared<G>* sh = reinterpret_cast<CondenseShared<G>*>(smem_raw) + slot_in_block;
-  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
-  const int64_t n = w.counts[kWaveRounds + 1];
-  const int nq = p.nq;
-  CondenseShared<G>& s = *sh;
-  for (int64_t i = (int64_t)blockIdx.x * epb + slot_in_block; i < n; i += (int64_t)gridDim.x * epb) {
-    const int64_t e = w.done[i];
-    Ctx<G, CondenseShared<G>> c{&p, sh, lane, mask, e, ne * nq, nullptr, nullptr, nullptr, nullptr, nullptr};
-    __syncwarp(mask);
-    if (lane < nq) {
-#pragma unroll
-      for (int f = 0; f < 12; ++f) s.geo[lane][f] = w.geo[(e * 12 + f) * G + lane];
-#pragma unroll 6
-      for (int f = 0; f < kSlot; ++f) s.slot[lane][f] = w.slot[(e * kSlot + f) * G + lane];
-    }
-    for (int k = lane; k < 9; k += G) {
-      s.jinv0[k] = w.jinv0[e * 9 + k];
-      s.rowp[k] = w.piv[e * 18 + k];
-      s.colp[k] = w.piv[e * 18 + 9 + k];
-    }
-    for (int k = lane; k < 81; k += G) s.lu[k] = w.kc[e * kKcStride + k];
-    for (int k = lane; k < 9; k += G) s.r[24 + k] = w.r[e * 33 + 24 + k];
-    c.sync();
-    force_sums(c);  // f_u and the energy of the last pass
-    condense<G, CondenseShared<G>, true>(c, want_tangent, force, tangent);
-    if (lane == 0) {
-      energy[e] = s.energy;
-      iterations[e] = w.iters[e];
-      code[e] = 0;
-    }
-    for (int k = lane; k < 9; k += G) alpha_out[e * 9 + k] = w.alpha[e * 9 + k];
   }
 }
 
@@ -3076,15 +2440,6 @@ int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t*
 
 namespace {
 
-// The next array of `count` T at byte offset `at` of base (256-byte
-// aligned); advances `at`. With a null base only the offsets are counted.
-template <class T>
-T* carve(char* base, size_t& at, size_t count) {
-  T* out = base ? reinterpret_cast<T*>(base + at) : nullptr;
-  at += (count * sizeof(T) + 255) / 256 * 256;
-  return out;
-}
-
 // The shared-memory limit of a kernel raised once per device, so that a
 // launch inside a stream capture makes no attribute call.
 template <class K>
@@ -3099,111 +2454,90 @@ int raise_smem(K kern, size_t smem, size_t* raised) {
   return 0;
 }
 
-}  // namespace
-
-namespace {
-
-size_t carve_all(char* base, int64_t ne, WaveBuffers& w) {
-  size_t at = 0;
-  const size_t n = (size_t)ne;
-  w.alpha = carve<double>(base, at, n * 9);
-  w.dir = carve<double>(base, at, n * 9);
-  w.res = carve<double>(base, at, n);
-  w.iters = carve<int32_t>(base, at, n);
-  w.pcode = carve<int32_t>(base, at, n);
-  w.kc = carve<double>(base, at, n * kKcStride);
-  w.r = carve<double>(base, at, n * 33);
-  w.sf = carve<double>(base, at, n * 19);
-  w.piv = carve<int32_t>(base, at, n * 18);
-  w.slot = carve<double>(base, at, n * kSlot * 8);
-  w.geo = carve<double>(base, at, n * 12 * 8);
-  w.jinv0 = carve<double>(base, at, n * 9);
-  w.hu = carve<double>(base, at, n * 9 * 8);
-  w.warm = carve<double>(base, at, n * 8 * 8);
-  w.pw = carve<double>(base, at, n * kPw * 8);
-  w.pfail = carve<int32_t>(base, at, n * 8);
-  w.pcodes = carve<int32_t>(base, at, n * 8);
-  w.plastic = carve<int32_t>(base, at, n * 8);
-  w.list[0] = carve<int32_t>(base, at, n);
-  w.list[1] = carve<int32_t>(base, at, n);
-  w.done = carve<int32_t>(base, at, n);
-  w.fallback = carve<int32_t>(base, at, n);
-  w.counts = carve<int32_t>(base, at, 2 * kWaveRounds + 3);
-  return at;
+// Elements of a full tile: the points of a block's threads, at most
+// kTileMostElements.
+int tile_most(int nq) {
+  const int n = kTileThreads / nq;
+  return n < kTileMostElements ? n : kTileMostElements;
 }
+constexpr int kTileBlocks = 148 * kTileBlocksPerSm;  // resident at once
+
+size_t aligned(size_t bytes) { return (bytes + 255) / 256 * 256; }
 
 }  // namespace
 
-size_t wave_buffer_bytes(int64_t ne) {
-  WaveBuffers w;
-  return carve_all(nullptr, ne, w);
+size_t tile_scratch_bytes(int64_t ne, int nq) {
+  const size_t points = (size_t)(tile_most(nq) * nq) | 1;
+  const int64_t blocks = ne < kTileBlocks ? ne : kTileBlocks;
+  return aligned(2 * sizeof(int32_t)) + aligned((size_t)ne * sizeof(int32_t)) +
+         aligned((size_t)blocks * kTileGeo * points * sizeof(double)) + 
+         (size_t)(ne < tile_chunk(nq) ? ne : tile_chunk(nq)) * cond_record(nq) * sizeof(double);
 }
 
-void wave_buffers_carve(void* base, int64_t ne, WaveBuffers& w) { carve_all(static_cast<char*>(base), ne, w); }
+void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s) {
+  char* at = static_cast<char*>(base);
+  s.counts = reinterpret_cast<int32_t*>(at);
+  at += aligned(2 * sizeof(int32_t));
+  s.fallback = reinterpret_cast<int32_t*>(at);
+  at += aligned((size_t)ne * sizeof(int32_t));
+  s.geo = reinterpret_cast<double*>(at);
+  const size_t points = (size_t)(tile_most(nq) * nq) | 1;
+  const int64_t blocks = ne < kTileBlocks ? ne : kTileBlocks;
+  at += aligned((size_t)blocks * kTileGeo * points * sizeof(double));
+  s.cond = reinterpret_cast<double*>(at);
+}
 
-bool wave_applies(const Params& p) { return p.element == 0 && p.nq <= 8; }
+bool tile_applies(const Params& p) { return p.element == 0; }
 
-int launch_elements_wave(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
+int launch_elements_tile(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
                          const double* state, const double* alpha_n, int want_tangent, double* force,
                          double* tangent, double* energy, double* trial, double* alpha_out, uint8_t* yield,
                          int32_t* iterations, int32_t* code, int32_t* first_failure, bool batch,
-                         const int32_t* order, const WaveBuffers& w, int pass_epb, cudaStream_t stream) {
-  constexpr int G = 8;
-  if (!wave_applies(p)) return (int)cudaErrorInvalidValue;
+                         const TileScratch& s, int elements_per_block, cudaStream_t stream) {
+  if (!tile_applies(p)) return (int)cudaErrorInvalidValue;
   if (ne <= 0) return 0;
-  constexpr int epb = 16;  // 4 warps per block
-  const int threads = epb * G;
-  // The first pass kernel's block: pass_epb elements (0: 16), at most 16
-  // (its launch bounds assume 128 threads).
-  const int pepb = pass_epb > 0 ? (pass_epb > 16 ? 16 : pass_epb) : 16;
-  static size_t raised[6][64] = {};
-  const size_t smem_pass = sizeof(PreShared<G>) * pepb;
-  const size_t smem_post = sizeof(PassShared<G>) * epb;
-  const size_t smem_ctl = sizeof(ControlShared<G>) * epb;
-  const size_t smem_cond = sizeof(CondenseShared<G>) * epb;
-  const size_t smem_elem = sizeof(ElemShared<G>) * epb;
-  auto pre = p.general ? wave_pre_kernel<G, true> : wave_pre_kernel<G, false>;
-  int rc = raise_smem(pre, smem_pass, raised[p.general ? 0 : 5]);
-  if (!rc) rc = raise_smem(wave_post_kernel<G>, smem_post, raised[4]);
-  if (!rc) rc = raise_smem(wave_control_kernel<G>, smem_ctl, raised[1]);
-  if (!rc) rc = raise_smem(wave_condense_kernel<G>, smem_cond, raised[2]);
-  if (!rc) rc = raise_smem(element_list_kernel<G>, smem_elem, raised[3]);
-  if (rc) return rc;
-  const int64_t need = (ne + epb - 1) / epb;
-  // Grid-stride launches: enough blocks to fill every SM several times over
-  // in the first rounds, few enough that the late rounds (a handful of
-  // elements) cost little more than the launch.
-  const int64_t cap = 148 * 16;
-  const unsigned grid = (unsigned)(need < cap ? need : cap);
-  const int64_t pneed = (ne + pepb - 1) / pepb;
-  const unsigned pgrid = (unsigned)(pneed < cap ? pneed : cap);
-  const int64_t rneed = (ne * 8 + 127) / 128;
-  const unsigned rgrid = (unsigned)(rneed < 148 * 8 ? rneed : 148 * 8);
-  const unsigned lgrid = rgrid;
-  cudaError_t err = cudaMemsetAsync(w.counts, 0, (2 * kWaveRounds + 3) * sizeof(int32_t), stream);
+  // A full tile per block once the mesh has that many elements; below, the
+  // elements spread evenly over the blocks that are resident at once.
+  const int most = tile_most(p.nq);
+  const int64_t even = (ne + kTileBlocks - 1) / kTileBlocks;
+  int elements = elements_per_block > 0 ? elements_per_block : (int)(even < most ? even : most);
+  if (elements > most) elements = most;
+  cudaError_t err = cudaMemsetAsync(s.counts + 1, 0, sizeof(int32_t), stream);
   if (err != cudaSuccess) return (int)err;
-  for (int r = 0; r < kWaveRounds; ++r) {
-    const int32_t* list = r == 0 ? order : w.list[r & 1];
-    const int32_t* count = r == 0 ? nullptr : w.counts + r;
-    int32_t* plastic_count = w.counts + kWaveRounds + 3 + r;
-    pre<<<pgrid, pepb * G, smem_pass, stream>>>(p, ne, r == 0, list, count, batch, coords, conn, u, state, alpha_n,
-                                                trial, yield, w.plastic, plastic_count, w);
-    launch_wave_returns(p, ne, w.plastic, plastic_count, state, trial, w, rgrid, stream);
-    if (p.kinematics == SBK_FINITE_LOGARITHMIC)
-      wave_log_kernel<<<lgrid, 128, 0, stream>>>(ne, p.nq, list, count, w);
-    wave_post_kernel<G><<<grid, threads, smem_post, stream>>>(p, ne, list, count, yield, w);
-    wave_control_kernel<G><<<grid, threads, smem_ctl, stream>>>(p, ne, r == 0, list, count, w, w.list[(r + 1) & 1],
-                                                                w.counts + r + 1, code, first_failure);
+  const int64_t chunk = tile_chunk(p.nq);
+  for (int64_t begin = 0; begin < ne; begin += chunk) {
+    const int64_t end = ne - begin < chunk ? ne : begin + chunk;
+    TileArgs a{ne, coords, conn, u, state, alpha_n, force, tangent, energy, trial, alpha_out, yield, iterations,
+               code, first_failure, want_tangent, batch ? 1 : 0, elements,
+               (int)((end - begin + elements - 1) / elements), begin, end};
+    const unsigned grid = (unsigned)(a.num_tiles < kTileBlocks ? a.num_tiles : kTileBlocks);
+    err = cudaMemsetAsync(s.counts, 0, sizeof(int32_t), stream);
+    if (err != cudaSuccess) return (int)err;
+    int rc;
+    if (!p.general) rc = launch_tile_j2(p, a, s, grid, stream);
+    else if (p.nterms == 0) rc = launch_tile_general0(p, a, s, grid, stream);
+    else if (p.nterms == 1) rc = launch_tile_general1(p, a, s, grid, stream);
+    else if (p.nterms == 2) rc = launch_tile_general2(p, a, s, grid, stream);
+    else rc = launch_tile_general4(p, a, s, grid, stream);
+    if (!rc) rc = launch_condense(p, a, s, stream);
+    if (rc) return rc;
   }
-  wave_condense_kernel<G><<<grid, threads, smem_cond, stream>>>(p, ne, w, want_tangent, force, tangent, energy,
-                                                                alpha_out, iterations, code);
   // The elements that left the common road, by the single kernel from the
-  // start (one 4-warp block per SM holds its records).
-  const unsigned fgrid = (unsigned)(need < 148 * 2 ? need : 148 * 2);
-  element_list_kernel<G><<<fgrid, threads, smem_elem, stream>>>(
-      p, ne, batch, coords, conn, u, state, alpha_n, want_tangent, force, tangent, energy, trial, alpha_out, yield,
-      iterations, code, first_failure, w.fallback, w.counts + kWaveRounds + 2);
-  return (int)cudaGetLastError();
+  // start (one block of it per SM).
+  auto list = [&](auto kern, int group, int epb, size_t record, size_t* raised) {
+    const size_t smem = record * epb;
+    const int bad = raise_smem(kern, smem, raised);
+    if (bad) return bad;
+    const int64_t need = (ne + epb - 1) / epb;
+    const unsigned blocks = (unsigned)(need < 148 * 2 ? need : 148 * 2);
+    kern<<<blocks, epb * group, smem, stream>>>(p, ne, batch, coords, conn, u, state, alpha_n, want_tangent, force,
+                                                tangent, energy, trial, alpha_out, yield, iterations, code,
+                                                first_failure, s.fallback, s.counts + 1);
+    return (int)cudaGetLastError();
+  };
+  static size_t raised[2][64] = {};
+  if (p.nq <= 8) return list(element_list_kernel<8>, 8, 16, sizeof(ElemShared<8>), raised[0]);
+  return list(element_list_kernel<32>, 32, 8, sizeof(ElemShared<32>), raised[1]);
 }
 
 size_t element_smem_bytes(int group) {

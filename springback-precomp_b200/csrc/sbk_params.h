@@ -37,6 +37,7 @@ struct Params {
   double PL[6];
   // Kinematic terms of the general return (Chaboche, then Prager).
   double termC[SBK_MAX_BACKSTRESSES], termG[SBK_MAX_BACKSTRESSES];
+  double termGi[SBK_MAX_BACKSTRESSES];  // 1 / termG (0 where that is 0)
   int nterms;       // terms stored per point (0 for the radial return)
   int general;      // 1: closest-point return (Hill48 and/or backstresses)
   int enabled;      // sy0 > 0

@@ -1,0 +1,88 @@
+// The tile kernel of the incompatible-mode Hex8 (sbk_tile.cuh): its launch
+// and its device scratch.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+#include "sbk_params.h"
+
+namespace sbk {
+
+// What the blocks of one launch keep in device memory: the tile counter, the
+// list of the elements that leave the common road, and per block the
+// geometry of its tile's points.
+struct TileScratch {
+  int32_t* counts;    // [0] next tile, [1] fallback elements
+  int32_t* fallback;  // ne
+  double* geo;        // blocks x kTileGeo x points of a tile
+  double* cond;       // tile_chunk x cond_record: the converged elements' records
+};
+
+// Where an evaluation reads and writes (launch_elements' arguments).
+struct TileArgs {
+  int64_t ne;
+  const double* coords;
+  const int32_t* conn;
+  const double* u;
+  const double* state;
+  const double* alpha_n;
+  double* force;
+  double* tangent;
+  double* energy;
+  double* trial;
+  double* alpha_out;
+  uint8_t* yield;
+  int32_t* iterations;
+  int32_t* code;
+  int32_t* first_failure;
+  int want_tangent;
+  int batch;
+  int elements;      // per tile
+  int num_tiles;
+  int64_t begin, end;  // the launch's elements
+};
+
+constexpr int kTileThreads = 256;
+constexpr int kTileBlocksPerSm = 1;
+constexpr int kTileMostElements = 32;
+constexpr int kTileGeo = 19;  // per point: J^-1 9, det0 / det, U G^T 9
+
+// A converged element's record for the condensation: per point, field-major
+// over the element's points, then the element's own values.
+constexpr int kCondH = 0;      // displacement gradient 9
+constexpr int kCondM = 9;      // material block 36
+constexpr int kCondS = 45;     // stress 6
+constexpr int kCondW = 51;     // w det J
+constexpr int kCondGeo = 52;   // J^-1 9, det0 / det
+constexpr int kCondPoint = 62;
+constexpr int kCondLu = 0;     // K_aa's factors 81, in pivot order
+constexpr int kCondPiv = 81;   // reciprocal pivots 9
+constexpr int kCondR = 90;     // r_a 9
+constexpr int kCondJ0 = 99;    // J0^-1 9
+constexpr int kCondPerm = 108; // 16 row + column of each pivot, 9
+constexpr int kCondElement = 118;
+__host__ __device__ inline size_t cond_record(int nq) { return (size_t)kCondPoint * nq + kCondElement; }
+
+// Elements of one launch: what 1 GiB of records holds (a mesh of more takes
+// several launches, so that the scratch does not grow with it).
+inline int64_t tile_chunk(int nq) { return (int64_t)((size_t(1) << 30) / (cond_record(nq) * sizeof(double))); }
+
+// The condensation of the launch's elements whose code is 0: force and,
+// wanted, K*.
+int launch_condense(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream);
+
+// Bytes of one allocation that tile_scratch_carve splits, for ne elements of
+// nq points.
+size_t tile_scratch_bytes(int64_t ne, int nq);
+void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s);
+
+// The tile kernel of the material's kind (one translation unit each).
+int launch_tile_j2(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
+int launch_tile_general0(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
+int launch_tile_general1(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
+int launch_tile_general2(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
+int launch_tile_general4(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
+
+}  // namespace sbk
