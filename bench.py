@@ -778,11 +778,10 @@ def run_cone(args, rank, world):
             "contact": {"begin_grid_ms": grid_ms, "begin_scan_ms": scan_ms, "candidates": grid_cand,
                         "active": [int(cev.tools[k][6]) for k in range(2)],
                         "slaves": [int(len(t["nodes"])) for t in prob.tools], "margin_m": margin},
-            # K1 (the tile kernel, the condensation, the single kernel's
-            # list), K2b + finish, K2a; per tool 7 contact
-            # kernels (moved points, evaluate, the ordered compaction's 3,
-            # scatter, resultants), the norms' two stages over both tools,
-            # and the blocks' add.
+            # K1 (the tile kernel, the condensation, the single kernel's list),
+            # K2b + finish, K2a; per tool 7 contact kernels (moved points,
+            # evaluate, the ordered compaction's 3, scatter, resultants), the
+            # norms' two stages over both tools, and the blocks' add.
             "gpu_launches": args.steps * (3 + 3 + 2 * 7 + 2 + 1), "clocks": clocks.summary(),
             "yielding_fraction": ev.yielding_points / (8.0 * ne),
             "setup_s": setup_s}
@@ -1152,7 +1151,7 @@ def main():
         el_ms = statistics.mean(elem_ms)
         # Kernels of one step: K1 (the tile kernel and the condensation per GiB
         # of records, 614 doubles an element, and the single kernel for the
-        # elements these leave; or one launch), then the force gather and its
+        # elements handed on; or one launch), then the force gather and its
         # finish (2), the value gather, and for the single kernel the schedule
         # (count, CUB's scan, place).
         phases = args.element == "incompatible_modes" and args.local_iteration == "phases"

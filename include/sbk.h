@@ -181,8 +181,8 @@ int sbk_system_set_elements_per_block(sbk_system* sys, int elements_per_block);
  * only in their last bits). SBK_LOCAL_PHASES (the default): one kernel over
  * tiles of elements, whose points and elements go through the phases of the
  * iteration together on chip, then the condensation of all elements; the
- * elements that need a line search, the shifted direction or
- * Levenberg-Marquardt are handed to the single kernel. Every rule.
+ * elements whose K_aa turns indefinite or whose line search fails are handed
+ * to the single kernel. Every rule.
  * SBK_LOCAL_SINGLE_KERNEL: one kernel runs each element from start to
  * finish. The first keeps records of up to 1 GiB on the device (4.9 KB an
  * element at 8 points, 10.9 KB at 20; allocated by the system when it is

@@ -740,21 +740,6 @@ __device__ __noinline__ void fullpiv_solve9_t(const double* lu, const int* rowp,
   for (int i = 0; i < 9; ++i) x[i] = y[i];
 }
 
-// Cholesky (lower, in place); false at the first non-positive pivot.
-__device__ __noinline__ bool llt9(double* a) {
-  _Pragma("unroll 1") for (int k = 0; k < 9; ++k) {
-    double x = a[k * 9 + k];
-    _Pragma("unroll 1") for (int j = 0; j < k; ++j) x -= a[k * 9 + j] * a[k * 9 + j];
-    if (x <= 0.0) return false;
-    a[k * 9 + k] = sqrt(x);
-    _Pragma("unroll 1") for (int i = k + 1; i < 9; ++i) {
-      double v = a[i * 9 + k];
-      _Pragma("unroll 1") for (int j = 0; j < k; ++j) v -= a[i * 9 + j] * a[k * 9 + j];
-      a[i * 9 + k] = v / a[k * 9 + k];
-    }
-  }
-  return true;
-}
 // llt9 by the lanes of a group together (every lane calls it): step k's
 // diagonal by the lane of row k, then the rows below in parallel, each entry
 // the same dot product in the same order - the same factor and the same
@@ -789,101 +774,6 @@ __device__ __forceinline__ bool llt9_rows_inline(const CT& c, double* a) {
 template <int G, class CT>
 __device__ __noinline__ bool llt9_rows(const CT& c, double* a) {
   return llt9_rows_inline<G>(c, a);
-}
-
-__device__ __noinline__ void llt9_solve(const double* l, const double* b, double* x) {
-  double y[9];
-  _Pragma("unroll 1") for (int i = 0; i < 9; ++i) {
-    double v = b[i];
-    _Pragma("unroll 1") for (int j = 0; j < i; ++j) v -= l[i * 9 + j] * y[j];
-    y[i] = v / l[i * 9 + i];
-  }
-  _Pragma("unroll 1") for (int i = 8; i >= 0; --i) {
-    double v = y[i];
-    _Pragma("unroll 1") for (int j = i + 1; j < 9; ++j) v -= l[j * 9 + i] * y[j];
-    y[i] = v / l[i * 9 + i];
-  }
-  _Pragma("unroll 1") for (int i = 0; i < 9; ++i) x[i] = y[i];
-}
-
-// Smallest eigenvalue and largest |eigenvalue| of a symmetric 9x9 (cyclic
-// Jacobi on a copy in `a`, destroyed).
-__device__ __noinline__ void sym_eig9(double* a, double* lo, double* top) {
-  _Pragma("unroll 1") for (int sweep = 0; sweep < 60; ++sweep) {
-    double off = 0.0, diag = 0.0;
-    _Pragma("unroll 1") for (int p = 0; p < 9; ++p) {
-      diag += a[p * 9 + p] * a[p * 9 + p];
-      _Pragma("unroll 1") for (int q = p + 1; q < 9; ++q) off += a[p * 9 + q] * a[p * 9 + q];
-    }
-    if (off == 0.0 || off <= 1.0e-36 * diag) break;
-    _Pragma("unroll 1") for (int p = 0; p < 8; ++p)
-      _Pragma("unroll 1") for (int q = p + 1; q < 9; ++q) {
-        const double apq = a[p * 9 + q];
-        if (apq == 0.0) continue;
-        const double theta = (a[q * 9 + q] - a[p * 9 + p]) / (2.0 * apq);
-        const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double cs = 1.0 / sqrt(t * t + 1.0);
-        const double sn = t * cs;
-        _Pragma("unroll 1") for (int k = 0; k < 9; ++k) {
-          const double akp = a[k * 9 + p], akq = a[k * 9 + q];
-          a[k * 9 + p] = cs * akp - sn * akq;
-          a[k * 9 + q] = sn * akp + cs * akq;
-        }
-        _Pragma("unroll 1") for (int k = 0; k < 9; ++k) {
-          const double apk = a[p * 9 + k], aqk = a[q * 9 + k];
-          a[p * 9 + k] = cs * apk - sn * aqk;
-          a[q * 9 + k] = sn * apk + cs * aqk;
-        }
-      }
-  }
-  double mn = a[0], mx = fabs(a[0]);
-  _Pragma("unroll 1") for (int i = 1; i < 9; ++i) {
-    mn = fmin(mn, a[i * 9 + i]);
-    mx = fmax(mx, fabs(a[i * 9 + i]));
-  }
-  *lo = mn;
-  *top = mx;
-}
-
-// Partial-pivoting LU solve of a 9x9 (in place), x = A^-1 b.
-__device__ __noinline__ void plu9_solve(double* a, int* perm, const double* b, double* x) {
-  _Pragma("unroll 1") for (int k = 0; k < 9; ++k) {
-    int p = k;
-    double big = fabs(a[k * 9 + k]);
-    _Pragma("unroll 1") for (int i = k + 1; i < 9; ++i)
-      if (fabs(a[i * 9 + k]) > big) {
-        big = fabs(a[i * 9 + k]);
-        p = i;
-      }
-    perm[k] = p;
-    if (big != 0.0) {
-      if (p != k)
-        _Pragma("unroll 1") for (int j = 0; j < 9; ++j) {
-          const double t = a[k * 9 + j];
-          a[k * 9 + j] = a[p * 9 + j];
-          a[p * 9 + j] = t;
-        }
-      const double inv = 1.0 / a[k * 9 + k];
-      _Pragma("unroll 1") for (int i = k + 1; i < 9; ++i) a[i * 9 + k] *= inv;
-    }
-    _Pragma("unroll 1") for (int i = k + 1; i < 9; ++i)
-      _Pragma("unroll 1") for (int j = k + 1; j < 9; ++j) a[i * 9 + j] -= a[i * 9 + k] * a[k * 9 + j];
-  }
-  double y[9];
-  _Pragma("unroll 1") for (int i = 0; i < 9; ++i) y[i] = b[i];
-  _Pragma("unroll 1") for (int k = 0; k < 9; ++k)
-    if (perm[k] != k) {
-      const double t = y[k];
-      y[k] = y[perm[k]];
-      y[perm[k]] = t;
-    }
-  _Pragma("unroll 1") for (int i = 1; i < 9; ++i)
-    _Pragma("unroll 1") for (int j = 0; j < i; ++j) y[i] -= a[i * 9 + j] * y[j];
-  _Pragma("unroll 1") for (int i = 8; i >= 0; --i) {
-    _Pragma("unroll 1") for (int j = i + 1; j < 9; ++j) y[i] -= a[i * 9 + j] * y[j];
-    y[i] /= a[i * 9 + i];
-  }
-  _Pragma("unroll 1") for (int i = 0; i < 9; ++i) x[i] = y[i];
 }
 
 // ---- the local iteration -------------------------------------------------------
@@ -2462,29 +2352,38 @@ int tile_most(int nq) {
 }
 constexpr int kTileBlocks = 148 * kTileBlocksPerSm;  // resident at once
 
-size_t aligned(size_t bytes) { return (bytes + 255) / 256 * 256; }
+}  // namespace
+
+namespace {
+
+// The arrays of a launch's scratch at base (NULL: their bytes only).
+size_t tile_layout(char* base, int64_t ne, int nq, TileScratch& s) {
+  const int most = tile_most(nq);
+  const size_t points = (size_t)(most * nq) | 1;
+  const size_t blocks = (size_t)(ne < kTileBlocks ? ne : kTileBlocks);
+  const size_t records = (size_t)(ne < tile_chunk(nq) ? ne : tile_chunk(nq));
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    char* here = base + at;
+    at += (bytes + 255) / 256 * 256;
+    return static_cast<void*>(here);
+  };
+  s.counts = static_cast<int32_t*>(take(2 * sizeof(int32_t)));
+  s.fallback = static_cast<int32_t*>(take((size_t)ne * sizeof(int32_t)));
+  s.geo = static_cast<double*>(take(blocks * kTileGeo * points * sizeof(double)));
+  s.cond = static_cast<double*>(take(records * cond_record(nq) * sizeof(double)));
+  return at;
+}
 
 }  // namespace
 
 size_t tile_scratch_bytes(int64_t ne, int nq) {
-  const size_t points = (size_t)(tile_most(nq) * nq) | 1;
-  const int64_t blocks = ne < kTileBlocks ? ne : kTileBlocks;
-  return aligned(2 * sizeof(int32_t)) + aligned((size_t)ne * sizeof(int32_t)) +
-         aligned((size_t)blocks * kTileGeo * points * sizeof(double)) + 
-         (size_t)(ne < tile_chunk(nq) ? ne : tile_chunk(nq)) * cond_record(nq) * sizeof(double);
+  TileScratch s;
+  return tile_layout(nullptr, ne, nq, s);
 }
 
 void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s) {
-  char* at = static_cast<char*>(base);
-  s.counts = reinterpret_cast<int32_t*>(at);
-  at += aligned(2 * sizeof(int32_t));
-  s.fallback = reinterpret_cast<int32_t*>(at);
-  at += aligned((size_t)ne * sizeof(int32_t));
-  s.geo = reinterpret_cast<double*>(at);
-  const size_t points = (size_t)(tile_most(nq) * nq) | 1;
-  const int64_t blocks = ne < kTileBlocks ? ne : kTileBlocks;
-  at += aligned((size_t)blocks * kTileGeo * points * sizeof(double));
-  s.cond = reinterpret_cast<double*>(at);
+  tile_layout(static_cast<char*>(base), ne, nq, s);
 }
 
 bool tile_applies(const Params& p) { return p.element == 0; }
@@ -2502,8 +2401,6 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
   const int64_t even = (ne + kTileBlocks - 1) / kTileBlocks;
   int elements = elements_per_block > 0 ? elements_per_block : (int)(even < most ? even : most);
   if (elements > most) elements = most;
-  cudaError_t err = cudaMemsetAsync(s.counts + 1, 0, sizeof(int32_t), stream);
-  if (err != cudaSuccess) return (int)err;
   const int64_t chunk = tile_chunk(p.nq);
   for (int64_t begin = 0; begin < ne; begin += chunk) {
     const int64_t end = ne - begin < chunk ? ne : begin + chunk;
@@ -2511,7 +2408,7 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
                code, first_failure, want_tangent, batch ? 1 : 0, elements,
                (int)((end - begin + elements - 1) / elements), begin, end};
     const unsigned grid = (unsigned)(a.num_tiles < kTileBlocks ? a.num_tiles : kTileBlocks);
-    err = cudaMemsetAsync(s.counts, 0, sizeof(int32_t), stream);
+    cudaError_t err = cudaMemsetAsync(s.counts, 0, (begin == 0 ? 2 : 1) * sizeof(int32_t), stream);
     if (err != cudaSuccess) return (int)err;
     int rc;
     if (!p.general) rc = launch_tile_j2(p, a, s, grid, stream);
@@ -2522,8 +2419,8 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
     if (!rc) rc = launch_condense(p, a, s, stream);
     if (rc) return rc;
   }
-  // The elements that left the common road, by the single kernel from the
-  // start (one block of it per SM).
+  // The elements handed on, by the single kernel from the start (one block of
+  // it per SM).
   auto list = [&](auto kern, int group, int epb, size_t record, size_t* raised) {
     const size_t smem = record * epb;
     const int bad = raise_smem(kern, smem, raised);

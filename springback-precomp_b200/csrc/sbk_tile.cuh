@@ -18,8 +18,10 @@
 //             the definiteness test.
 //
 // Then the states and energies, a thread a point; what the condensation takes
-// goes to condense_kernel (sbk_condense.cu). An element whose step needs a line search, the shifted direction or
-// Levenberg-Marquardt goes to the fallback list (element_list_kernel).
+// goes to condense_kernel (sbk_condense.cu). An element whose full Newton step
+// is refused goes on in the same rounds, its line search's trial a trial like
+// any other (sbk_tile_search.cuh); one whose K_aa is indefinite or whose line
+// search fails goes to the single kernel (element_list_kernel).
 //
 // Why: as one launch per stage over the whole mesh (130 launches) the stages
 // handed each other 207 KB per element through DRAM, and a mesh of a few
@@ -45,6 +47,7 @@
 #include "sbk_element_math.cuh"
 #include "sbk_tile.h"
 #include "sbk_tile_point.cuh"
+#include "sbk_tile_search.cuh"
 
 namespace sbk {
 
@@ -62,11 +65,14 @@ constexpr int kRec = 84;
 struct TileElement {
   double kc[81];    // K_aa of the last pass; of a converged element its LU
   double r[9], scale[9], flo[9];
-  double alpha[9], at[9], dir[9], jinv0[9], ipiv[9];
+  double alpha[9], at[9], jinv0[9], ipiv[9];
+  double dir[9], r0[9];  // the direction of the trials, r_a where it starts
   double res;
   int64_t e;
   int fail;         // (stage << 16) | (point << 8) | code of the first failure
   int iterations;
+  int stage;        // what the pending trial is (sbk_tile_search.cuh)
+  TileSearch search;
   uint8_t rowp[12], colp[12];
 };
 
@@ -380,18 +386,17 @@ struct Tile {
   }
 
   // What follows a pass of element k (solve_and_condense's loop,
-  // IncompatibleModes.cpp:353-397, and the full step of its line search), by
-  // 16 lanes, lane i < 9 the row i of K_aa; both halves of a warp walk it
-  // together (a shuffle under a mask known only at run time costs several
-  // instructions more). Returns 0: the element goes on with the trial modes
-  // `at`; 1: converged; 2: for the fallback; -1: not live; else its failure
-  // << 8.
+  // IncompatibleModes.cpp:353-546), by 16 lanes, lane i < 9 the row i of
+  // K_aa; both halves of a warp walk it together (a shuffle under a mask
+  // known only at run time costs several instructions more). Returns 0: the
+  // element goes on with the trial modes `at`; 1: converged; 2: handed to the
+  // single kernel; -1: not live; else its failure << 8.
   __device__ __forceinline__ int control(int k, bool live, bool first, int lane) {
     TileElement& E = el[k];
     const int fail = live ? E.fail : 0;
     const bool row = lane < 9;
-    double b = row ? E.r[lane] : 0.0;
-    double full = b * b, largest = fabs(b), scale = row ? fabs(E.scale[lane]) : 0.0,
+    const double r = row ? E.r[lane] : 0.0;
+    double b = r, full = b * b, largest = fabs(b), scale = row ? fabs(E.scale[lane]) : 0.0,
            floors = row ? fabs(E.flo[lane]) : 0.0;
 #pragma unroll
     for (int o = 8; o >= 1; o >>= 1) {
@@ -402,12 +407,25 @@ struct Tile {
     }
     full = sqrt(full);
     const double bound = kLocalTolerance * scale + kLocalRoundOff * floors;
+    // The full Newton step, accepted when it reduces the residual enough or
+    // meets the tolerance; everything else is search_after's.
+    const bool evaluated = fail == 0x7fffffff;
+    const bool reduced = evaluated && (full <= kFullStepReduction * E.res || largest <= bound);
     int out = -1;
-    if (live) {
-      if (fail != 0x7fffffff) out = first ? (fail & 0xff) << 8 : 2;
-      else if (!first && !(full <= kFullStepReduction * E.res || largest <= bound)) out = 2;
+    bool go = live && (first ? evaluated : E.stage == kStageNewton && reduced);
+    if (live && first && !evaluated) out = (fail & 0xff) << 8;
+    const bool look = live && !first && !go;
+    if (__any_sync(kAll, look)) {
+      int got = 0;
+      if (look && lane == 0)
+        got = search_after(E, E.search, evaluated, full, largest <= bound, full <= kFullStepReduction * E.res);
+      got = __shfl_sync(kAll, got, 0, 16);
+      __syncwarp();
+      if (look) {
+        go = got == 1;
+        if (!go) out = got;
+      }
     }
-    const bool go = live && out == -1;  // the trial is accepted
     if (!__any_sync(kAll, go)) return out;
     // K_aa = L U without exchanges, the right-hand side eliminated beside
     // it, and the symmetric part's L D L^T for the definiteness test (for a
@@ -451,14 +469,14 @@ struct Tile {
     const bool converged = largest <= bound || largest == 0.0;
     // Definite and far from singular: no pivot search is needed. Anything
     // else takes the complete pivoting and its rank test.
-    const bool search = go && !(positive && small_pivot > 1.0e-10 * big_pivot);
-    if (__any_sync(kAll, search)) {
-      const int got = pivoted(E, search, largest, converged, lane);
-      if (search) out = got;
-    }
-    if (go && !search) {
-      if (converged) {
-        if (row) {
+    const bool pivot = go && !(positive && small_pivot > 1.0e-10 * big_pivot);
+    int status = -1;
+    if (__any_sync(kAll, pivot)) status = pivoted(E, pivot, r, converged, lane);
+    if (go) {
+      if (pivot && status) {
+        out = SBK_EL_LOCAL_SINGULAR << 8;
+      } else if (converged) {
+        if (!pivot && row) {
           E.rowp[lane] = E.colp[lane] = (uint8_t)lane;
           E.ipiv[lane] = myinv;
 #pragma unroll
@@ -466,10 +484,11 @@ struct Tile {
         }
         out = 1;
       } else {
-        out = E.iterations == kMaxLocal || !isfinite(largest) ? SBK_EL_LOCAL_NO_CONVERGE << 8 : 0;
+        out = E.iterations == kMaxLocal || !isfinite(largest) ? SBK_EL_LOCAL_NO_CONVERGE << 8 : (positive ? 0 : 2);
       }
     }
-    if (!__any_sync(kAll, out == 0)) return out;
+    const bool on = go && out == 0;
+    if (!__any_sync(kAll, on)) return out;
     double x = 0.0;
 #pragma unroll
     for (int s = 8; s >= 0; --s) {
@@ -477,25 +496,31 @@ struct Tile {
       if (lane == s) x = xs;
       b -= lane < s ? A[s] * xs : 0.0;
     }
-    if (out == 0) {
-      if (row) E.at[lane] = E.alpha[lane] - x;
+    if (on) {
+      if (row) {
+        const double d = pivot ? E.dir[lane] : -x;  // pivoted leaves its own
+        E.dir[lane] = d;
+        E.r0[lane] = r;
+        E.at[lane] = E.alpha[lane] + d;
+      }
       if (lane == 0) {
         E.iterations += 1;
         E.res = full;
+        E.stage = kStageNewton;
       }
     }
     return out;
   }
 
   // control's step with complete pivoting (Eigen's FullPivLU and its rank
-  // test). No row or column moves: a lane knows its row's step, a mask the
-  // columns that are done. An element that goes on from here has an
-  // indefinite symmetric part or a K_aa close to singular: the fallback's
-  // business. Both halves of the warp walk it; `need`: this one's outcome
-  // counts.
-  __device__ __noinline__ static int pivoted(TileElement& E, bool need, double largest, bool converged, int lane) {
+  // test), both halves of the warp together; `need`: this one's outcome
+  // counts. No row or column moves: a lane knows its row's step, a mask the
+  // columns that are done. Returns 1 for a singular K_aa; else the factors
+  // of a converged element are in its record, or minus the solution for r
+  // in dir.
+  __device__ __noinline__ static int pivoted(TileElement& E, bool need, double r, bool converged, int lane) {
     const bool row = lane < 9;
-    double A[9];
+    double A[9], b = r;
 #pragma unroll
     for (int j = 0; j < 9; ++j) A[j] = row ? E.kc[lane * 9 + j] : 0.0;
     __syncwarp();
@@ -534,12 +559,13 @@ struct Tile {
       const double l0 = pick9(A, pc);
       const double inv = 1.0 / __shfl_sync(kAll, l0, pr, 16);
       const bool below = mystep == 9 && lane != pr;
-      const double l = l0 * inv;
+      const double l = below ? l0 * inv : 0.0;
 #pragma unroll
       for (int j = 0; j < 9; ++j) {
         const double u = __shfl_sync(kAll, A[j], pr, 16);
         if (below && !((done >> j) & 1u)) A[j] = j == pc ? l : A[j] - l * u;
       }
+      b -= l * __shfl_sync(kAll, b, pr, 16);
       if (lane == pr && mystep == 9) {
         mystep = s;
         myinv = inv;
@@ -548,24 +574,26 @@ struct Tile {
       ro |= (uint64_t)pr << (4 * s);
       co |= (uint64_t)pc << (4 * s);
     }
-    if (singular || !(small_pivot > kEps * 9.0 * big_pivot)) return SBK_EL_LOCAL_SINGULAR << 8;
-    if (converged) {
-      if (row && need) {
-        E.rowp[lane] = (uint8_t)((ro >> (4 * lane)) & 15);
-        E.colp[lane] = (uint8_t)((co >> (4 * lane)) & 15);
-        E.ipiv[mystep] = myinv;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-          int step = 0;
-#pragma unroll
-          for (int s = 0; s < 9; ++s) step = (int)((co >> (4 * s)) & 15) == j ? s : step;
-          E.kc[mystep * 9 + step] = A[j];
-        }
-      }
-      return 1;
+    double x = 0.0;
+#pragma unroll 1
+    for (int s = 8; s >= 0; --s) {
+      const int pr = (int)((ro >> (4 * s)) & 15), pc = (int)((co >> (4 * s)) & 15);
+      const double xs = __shfl_sync(kAll, b * myinv, pr, 16);
+      if (lane == pc) x = xs;
+      if (mystep < s) b -= pick9(A, pc) * xs;
     }
-    if (E.iterations == kMaxLocal || !isfinite(largest)) return SBK_EL_LOCAL_NO_CONVERGE << 8;
-    return 2;
+    if (singular || !(small_pivot > kEps * 9.0 * big_pivot)) return 1;
+    if (!need || !row) return 0;
+    if (converged) {
+      E.rowp[lane] = (uint8_t)((ro >> (4 * lane)) & 15);
+      E.colp[lane] = (uint8_t)((co >> (4 * lane)) & 15);
+      E.ipiv[mystep] = myinv;
+#pragma unroll 1
+      for (int s = 0; s < 9; ++s) E.kc[mystep * 9 + s] = pick9(A, (int)((co >> (4 * s)) & 15));
+    } else {
+      E.dir[lane] = -x;
+    }
+    return 0;
   }
 };
 
@@ -689,6 +717,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSm)
         const int k = active[side][live ? i >> 4 : 0];
         const int out = T.control(k, live, round == 0, i & 15);
         if ((i & 15) == 0 && live) {
+          T.el[k].fail = 0x7fffffff;  // a trial's failure is its search's
           if (out == 0) {
             active[side ^ 1][atomicAdd(&count[side ^ 1], 1)] = (int8_t)k;
           } else if (out == 1) {

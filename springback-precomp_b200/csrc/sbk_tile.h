@@ -10,11 +10,17 @@
 
 namespace sbk {
 
+// An element's line search (sbk_tile_search.cuh).
+struct TileSearch {
+  double phi0, reach, s0, f0, s1, f1, step, best, best_step;
+  int count, halvings, side, last_is_best;
+};
+
 // What the blocks of one launch keep in device memory: the tile counter, the
-// list of the elements that leave the common road, and per block the
+// list of the elements handed to the single kernel, and per block the
 // geometry of its tile's points.
 struct TileScratch {
-  int32_t* counts;    // [0] next tile, [1] fallback elements
+  int32_t* counts;    // [0] the next tile, [1] elements handed on
   int32_t* fallback;  // ne
   double* geo;        // blocks x kTileGeo x points of a tile
   double* cond;       // tile_chunk x cond_record: the converged elements' records

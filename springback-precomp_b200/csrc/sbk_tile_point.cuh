@@ -88,13 +88,30 @@ __device__ __forceinline__ void rotate_out(const double q[9], const double a[6],
 // E_log (engineering Voigt) of a Green-Lagrange strain (engineering Voigt)
 // and its spectral data L. L.q holds the axes to start from: those of the
 // element's last pass, in which the strain of the next is nearly diagonal (a
-// sweep or two remain of four or five), or the identity.
+// sweep or two remain of four or five), or the identity. One step of Newton's
+// iteration for the nearest orthogonal matrix, Q (3 - Q^T Q) / 2, first: each
+// pass's rotations leave them off by some units in the last place, which
+// would add up over an element's passes.
 __device__ __forceinline__ int spectral_log(const double green[6], LogKin& L, double elog[6]) {
 #pragma unroll
   for (int i = 0; i < 6; ++i)
     if (!isfinite(green[i])) return kFailNonFinite;
   double a[6];
   {
+    double g[6], q[9];  // (3 - Q^T Q) / 2
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int i = k < 3 ? k : k - 3, j = k < 3 ? k : (k - 2) % 3;
+      g[k] = (i == j ? 1.5 : 0.0) - 0.5 * (L.q[i] * L.q[j] + L.q[3 + i] * L.q[3 + j] + L.q[6 + i] * L.q[6 + j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      q[3 * i] = L.q[3 * i] * g[0] + L.q[3 * i + 1] * g[3] + L.q[3 * i + 2] * g[5];
+      q[3 * i + 1] = L.q[3 * i] * g[3] + L.q[3 * i + 1] * g[1] + L.q[3 * i + 2] * g[4];
+      q[3 * i + 2] = L.q[3 * i] * g[5] + L.q[3 * i + 1] * g[4] + L.q[3 * i + 2] * g[2];
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) L.q[i] = q[i];
     const double e[6] = {green[0], green[1], green[2], 0.5 * green[3], 0.5 * green[4], 0.5 * green[5]};
     rotate_in(L.q, e, a);
   }
@@ -346,20 +363,22 @@ __device__ __forceinline__ bool point_window(const Params& p, const PointTrial<N
 //   r_k = y_k (1 + f L_k) - z_k(dl),  f = b / sigma_bar,
 //   r_7 = sigma_bar - sigma_y(a_n + dl),
 // with z(dl) the trial relative stress: no 6 x 6 product is left in the
-// iteration. With n = L y / sigma_bar, d = 1 / (1 + f L) and the Jacobian
-// [[diag(1 + f L) - f n n^T, j], [n^T, -h]], j = back_rate + db n, the rank
-// one term goes by Sherman-Morrison, the border by its Schur complement. The
-// consistent tangent closes to one diagonal and one rank-one term,
-//   C_alg = C^e - 4 G^2 [g V diag(L d) V^T + (V u) (V bm)^T],
-// g = dl / sigma_bar, bm = d n, kappa = 1 / (1 - f n.bm), c = f kappa,
-// u = g c L bm + (kappa / s) ((1 - g h) n - g L aj), aj = A^-1 j and s =
-// n.aj + h (n.x = h y_7 removes the other products).
+// iteration. With n = L y / sigma_bar, d = 1 / (1 + f L), bm = d n and the
+// Jacobian [[diag(1 + f L) - f n n^T, j], [n^T, -h]], j = back_rate + db n,
+// the rank one term goes by Sherman-Morrison (kappa = 1 / (1 - f n.bm) = 1 /
+// sum n y d / sigma_bar, as sum n^2 / L = 1), the border by its Schur
+// complement s = kappa bm.j + h. The consistent tangent, from the stress as y
+// plus the back stresses, closes to one diagonal and one rank-one term in
+// which nothing of the elastic modulus's size cancels but their sum:
+//   C_alg = lambda 1 1^T + 2 G V diag((1 + f_k L) d) V^T + 2 G (V w) (V bm)^T,
+//   w = 2 G (kappa / s) d {g L back_rate + n [g (h + db_k L) - (1 + f_k L)]},
+// with g = dl / sigma_bar and f_k, db_k the kinematic terms' shares of f, db.
 
 struct ReturnPoint {
   double y[6], dl;
   double inv;          // 1 / sigma_bar
   double n[6];         // L y / sigma_bar
-  double b, db;        // 2G dl + 2/3 sum C chi, and its derivative
+  double bk, b, db;    // 2/3 sum C chi; with 2G dl; its derivative
   double back_rate[6];
   double res[7];
   double slope;        // sigma_y'(a_n + dl)
@@ -435,7 +454,7 @@ __device__ __forceinline__ bool return_evaluate(const Params& p, const ReturnTri
     z[k] = T.s[k];
     e.back_rate[k] = 0.0;
   }
-  e.b = 2.0 * p.G * e.dl;
+  e.bk = 0.0;
   e.db = 2.0 * p.G;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -447,10 +466,11 @@ __device__ __forceinline__ bool return_evaluate(const Params& p, const ReturnTri
         z[k] -= theta * T.a[t][k];
         e.back_rate[k] += dtheta * T.a[t][k];
       }
-      e.b += 2.0 / 3.0 * p.termC[t] * chi;
+      e.bk += 2.0 / 3.0 * p.termC[t] * chi;
       e.db += 2.0 / 3.0 * p.termC[t] * dchi;
     }
   }
+  e.b = e.bk + 2.0 * p.G * e.dl;
 #pragma unroll
   for (int k = 0; k < 6; ++k) e.res[k] = e.y[k] - z[k] + e.b * e.n[k];
   const double a = T.a_n + e.dl;
@@ -475,7 +495,7 @@ __device__ __forceinline__ double return_norm2(const ReturnPoint& e) {
 
 struct ReturnFactor {
   double d[6], bm[6], aj[6];
-  double kappa, c, si;  // 1 / (1 - f n.bm), f kappa, 1 / (n.aj + h)
+  double kappa, c, si;  // kappa, f kappa, 1 / s
 };
 
 __device__ __forceinline__ double dot6(const double a[6], const double b[6]) {
@@ -489,30 +509,29 @@ __device__ __forceinline__ void return_factor(const Params& p, const ReturnPoint
     r.d[k] = 1.0 / (1.0 + f * p.PL[k]);
     r.bm[k] = r.d[k] * e.n[k];
   }
-  r.kappa = 1.0 / (1.0 - f * dot6(e.n, r.bm));
+  r.kappa = 1.0 / (e.inv * dot6(r.bm, e.y));
   r.c = f * r.kappa;
   double j[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) j[k] = e.back_rate[k] + e.db * e.n[k];
-  const double g = r.c * dot6(r.bm, j);
+  const double bj = dot6(r.bm, j);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) r.aj[k] = r.d[k] * j[k] + g * r.bm[k];
-  r.si = 1.0 / (dot6(e.n, r.aj) + e.slope);
+  for (int k = 0; k < 6; ++k) r.aj[k] = r.d[k] * j[k] + r.c * bj * r.bm[k];
+  r.si = 1.0 / (r.kappa * bj + e.slope);
 }
 
 // C_alg into the record.
 __device__ __forceinline__ void return_tangent(const Params& p, const ReturnPoint& e, const ReturnFactor& r,
                                                const PointRecord& rec, int fM) {
-  const double g2 = 4.0 * p.G * p.G;
-  const double g = e.dl * e.inv;
-  double u[6], w[6], vb[6];
-  const double ks = r.kappa * r.si;
+  const double g = e.dl * e.inv, fk = e.bk * e.inv, dbk = e.db - 2.0 * p.G;
+  const double g2 = 2.0 * p.G, ks = g2 * g2 * r.kappa * r.si;
+  double u[6], w[6], vu[6], vb[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    u[k] = g * r.c * p.PL[k] * r.bm[k] + ks * ((1.0 - g * e.slope) * e.n[k] - g * p.PL[k] * r.aj[k]);
-    w[k] = g2 * g * p.PL[k] * r.d[k];
+    const double l = p.PL[k], kin = 1.0 + fk * l;
+    w[k] = g2 * (kin * r.d[k]);
+    u[k] = ks * r.d[k] * (g * l * e.back_rate[k] + e.n[k] * (g * (e.slope + dbk * l) - kin));
   }
-  double vu[6];
   from_basis(p, u, vu);
   from_basis(p, r.bm, vb);
   const double lame = p.K - 2.0 * p.G / 3.0;
@@ -523,9 +542,9 @@ __device__ __forceinline__ void return_tangent(const Params& p, const ReturnPoin
       double v = 0.0;
 #pragma unroll
       for (int k = 0; k < 6; ++k) v += w[k] * p.PV[i * 6 + k] * p.PV[j * 6 + k];
-      const double el = i < 3 ? (j < 3 ? lame : 0.0) + (i == j ? 2.0 * p.G : 0.0) : (i == j ? p.G : 0.0);
-      rec.put(fM + i * 6 + j, el - v - g2 * vu[i] * vb[j]);
-      if (i != j) rec.put(fM + j * 6 + i, el - v - g2 * vu[j] * vb[i]);
+      if (i < 3 && j < 3) v += lame;
+      rec.put(fM + i * 6 + j, v + vu[i] * vb[j]);
+      if (i != j) rec.put(fM + j * 6 + i, v + vu[j] * vb[i]);
     }
 }
 

@@ -304,8 +304,7 @@ class NonlinearSystem:
     def set_local_iteration(self, mode: str = "phases"):
         """How the incompatible-mode Hex8's local iteration runs: "phases"
         (the default: tiles of elements through the iteration's phases
-        together, the elements that need a line search or a fallback handed
-        to the single kernel) or
+        together) or
         "single" (one kernel per element from start to finish). No result
         depends on it."""
         _capi.check(_capi.lib().sbk_system_set_local_iteration(self._h, LOCAL_ITERATION[mode]))
