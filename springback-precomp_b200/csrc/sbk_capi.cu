@@ -972,11 +972,14 @@ int sbk_system_vjp_x(sbk_system* sys, const double* u_dev, const double* lambda_
   cudaStream_t st = sys->stream;
   Params p = sys->p;
   if (frozen) p.enabled = 0;  // the committed plastic state, no return
+  int rc = ensure_tile(sys);  // there already unless the system was made for the single kernel
+  if (rc) return rc;
   SBK_CUDA(cudaMemsetAsync(sys->first_fail, 0x7f, sizeof(int32_t), st));
   sys->has_trial = false;  // the trial buffers are overwritten
-  int rc = sbk::launch_vjp(p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c, lambda_dev,
-                           sys->trial, sys->yield, sys->code, sys->first_fail, sys->force, st);
-  if (rc) return rc;
+  rc = sbk::launch_vjp(p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c, lambda_dev,
+                       sys->energy_e, sys->trial, sys->alpha_t, sys->yield, sys->iters, sys->code, sys->first_fail,
+                       sys->force, sys->tile, sys->elements_per_block, st);
+  if (rc) return fail(SBK_ERR_CUDA, std::string("shape derivative: ") + cudaGetErrorString((cudaError_t)rc));
   int32_t first = 0;
   SBK_CUDA(cudaMemcpyAsync(&first, sys->first_fail, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   SBK_CUDA(cudaStreamSynchronize(st));

@@ -1440,22 +1440,13 @@ __device__ __noinline__ void vjp_point(const Ctx<G>& c, int q, const double* lam
 }
 
 template <int G>
-__global__ void __launch_bounds__(256) vjp_kernel(const __grid_constant__ Params p, int64_t ne,
-                                                  const double* __restrict__ coords, const int32_t* __restrict__ conn,
-                                                  const double* __restrict__ u, const double* __restrict__ state,
-                                                  const double* __restrict__ alpha_n,
-                                                  const double* __restrict__ lambda, double* __restrict__ trial,
-                                                  uint8_t* __restrict__ yield, int32_t* __restrict__ code,
-                                                  int32_t* __restrict__ first_failure, double* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int epb = blockDim.x / G;
-  const int slot_in_block = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  const int64_t e = (int64_t)blockIdx.x * epb + slot_in_block;
-  ElemShared<G>* sh = reinterpret_cast<ElemShared<G>*>(smem_raw) + slot_in_block;
-  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
-  if (e >= ne) return;
+__device__ __forceinline__ void vjp_element(const Params& p, int64_t ne, int64_t e, ElemShared<G>* sh, int lane,
+                                            unsigned mask, const double* __restrict__ coords,
+                                            const int32_t* __restrict__ conn, const double* __restrict__ u,
+                                            const double* __restrict__ state, const double* __restrict__ alpha_n,
+                                            const double* __restrict__ lambda, double* __restrict__ trial,
+                                            uint8_t* __restrict__ yield, int32_t* __restrict__ code,
+                                            int32_t* __restrict__ first_failure, double* __restrict__ out) {
   double hu_lane[9];
   double warm_lane[8];
   warm_lane[7] = 0.0;
@@ -1570,6 +1561,32 @@ __global__ void __launch_bounds__(256) vjp_kernel(const __grid_constant__ Params
                                 red[24 + i * 3 + 2] * dn0[2];
   }
   if (lane == 0) code[e] = 0;
+}
+
+// The elements the tile kernel handed on (grid-stride over its list).
+template <int G>
+__global__ void __launch_bounds__(256) vjp_kernel(const __grid_constant__ Params p, int64_t ne,
+                                                  const double* __restrict__ coords, const int32_t* __restrict__ conn,
+                                                  const double* __restrict__ u, const double* __restrict__ state,
+                                                  const double* __restrict__ alpha_n,
+                                                  const double* __restrict__ lambda, double* __restrict__ trial,
+                                                  uint8_t* __restrict__ yield, int32_t* __restrict__ code,
+                                                  int32_t* __restrict__ first_failure, double* __restrict__ out,
+                                                  const int32_t* __restrict__ list,
+                                                  const int32_t* __restrict__ count) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int epb = blockDim.x / G;
+  const int slot_in_block = threadIdx.x / G;
+  const int lane = threadIdx.x % G;
+  ElemShared<G>* sh = reinterpret_cast<ElemShared<G>*>(smem_raw) + slot_in_block;
+  const unsigned lanes_mask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
+  const unsigned mask = lanes_mask << ((threadIdx.x % 32) / G * G);
+  const int64_t n = *count;
+  for (int64_t i = (int64_t)blockIdx.x * epb + slot_in_block; i < n; i += (int64_t)gridDim.x * epb) {
+    __syncwarp(mask);
+    vjp_element<G>(p, ne, (int64_t)list[i], sh, lane, mask, coords, conn, u, state, alpha_n, lambda, trial, yield,
+                   code, first_failure, out);
+  }
 }
 
 // ---- the standard Hex8 -------------------------------------------------------
@@ -2300,34 +2317,6 @@ int launch_standard_g(const Params& p, int64_t ne, const double* coords, const i
   return 0;
 }
 
-template <int G>
-int launch_vjp_g(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
-                 const double* state, const double* alpha_n, const double* lambda, double* trial, uint8_t* yield,
-                 int32_t* code, int32_t* first_failure, double* out, cudaStream_t stream) {
-  const int epb = G == 8 ? 16 : 4;
-  const size_t smem = sizeof(ElemShared<G>) * epb;
-  const int64_t blocks = (ne + epb - 1) / epb;
-  if (blocks == 0) return 0;
-  auto kern = vjp_kernel<G>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return set_error(SBK_ERR_CUDA, std::string("vjp kernel attribute: ") + cudaGetErrorString(err));
-  kern<<<(unsigned)blocks, epb * G, smem, stream>>>(p, ne, coords, conn, u, state, alpha_n, lambda, trial, yield, code,
-                                                    first_failure, out);
-  err = cudaGetLastError();
-  if (err != cudaSuccess) return set_error(SBK_ERR_CUDA, std::string("vjp kernel launch: ") + cudaGetErrorString(err));
-  return 0;
-}
-
-int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
-               const double* state, const double* alpha_n, const double* lambda, double* trial, uint8_t* yield,
-               int32_t* code, int32_t* first_failure, double* out, cudaStream_t stream) {
-  if (p.nq <= 8)
-    return launch_vjp_g<8>(p, ne, coords, conn, u, state, alpha_n, lambda, trial, yield, code, first_failure, out,
-                           stream);
-  return launch_vjp_g<32>(p, ne, coords, conn, u, state, alpha_n, lambda, trial, yield, code, first_failure, out,
-                          stream);
-}
-
 namespace {
 
 // The shared-memory limit of a kernel raised once per device, so that a
@@ -2388,27 +2377,26 @@ void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s) {
 
 bool tile_applies(const Params& p) { return p.element == 0; }
 
-int launch_elements_tile(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
-                         const double* state, const double* alpha_n, int want_tangent, double* force,
-                         double* tangent, double* energy, double* trial, double* alpha_out, uint8_t* yield,
-                         int32_t* iterations, int32_t* code, int32_t* first_failure, bool batch,
-                         const TileScratch& s, int elements_per_block, cudaStream_t stream) {
+namespace {
+
+// The tile kernel over the elements of `a`, in launches of tile_chunk, each
+// followed by after(its arguments, its scratch).
+template <class After>
+int run_tiles(const Params& p, TileArgs a, const TileScratch& s, int elements_per_block, cudaStream_t stream,
+              After after) {
   if (!tile_applies(p)) return (int)cudaErrorInvalidValue;
-  if (ne <= 0) return 0;
   // A full tile per block once the mesh has that many elements; below, the
   // elements spread evenly over the blocks that are resident at once.
   const int most = tile_most(p.nq);
-  const int64_t even = (ne + kTileBlocks - 1) / kTileBlocks;
-  int elements = elements_per_block > 0 ? elements_per_block : (int)(even < most ? even : most);
-  if (elements > most) elements = most;
+  const int64_t even = (a.ne + kTileBlocks - 1) / kTileBlocks;
+  a.elements = elements_per_block > 0 ? elements_per_block : (int)(even < most ? even : most);
+  if (a.elements > most) a.elements = most;
   const int64_t chunk = tile_chunk(p.nq);
-  for (int64_t begin = 0; begin < ne; begin += chunk) {
-    const int64_t end = ne - begin < chunk ? ne : begin + chunk;
-    TileArgs a{ne, coords, conn, u, state, alpha_n, force, tangent, energy, trial, alpha_out, yield, iterations,
-               code, first_failure, want_tangent, batch ? 1 : 0, elements,
-               (int)((end - begin + elements - 1) / elements), begin, end};
+  for (a.begin = 0; a.begin < a.ne; a.begin += chunk) {
+    a.end = a.ne - a.begin < chunk ? a.ne : a.begin + chunk;
+    a.num_tiles = (int)((a.end - a.begin + a.elements - 1) / a.elements);
     const unsigned grid = (unsigned)(a.num_tiles < kTileBlocks ? a.num_tiles : kTileBlocks);
-    cudaError_t err = cudaMemsetAsync(s.counts, 0, (begin == 0 ? 2 : 1) * sizeof(int32_t), stream);
+    cudaError_t err = cudaMemsetAsync(s.counts, 0, (a.begin == 0 ? 2 : 1) * sizeof(int32_t), stream);
     if (err != cudaSuccess) return (int)err;
     int rc;
     if (!p.general) rc = launch_tile_j2(p, a, s, grid, stream);
@@ -2416,25 +2404,64 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
     else if (p.nterms == 1) rc = launch_tile_general1(p, a, s, grid, stream);
     else if (p.nterms == 2) rc = launch_tile_general2(p, a, s, grid, stream);
     else rc = launch_tile_general4(p, a, s, grid, stream);
-    if (!rc) rc = launch_condense(p, a, s, stream);
+    if (!rc) rc = after(a);
     if (rc) return rc;
   }
-  // The elements handed on, by the single kernel from the start (one block of
-  // it per SM).
-  auto list = [&](auto kern, int group, int epb, size_t record, size_t* raised) {
-    const size_t smem = record * epb;
-    const int bad = raise_smem(kern, smem, raised);
-    if (bad) return bad;
-    const int64_t need = (ne + epb - 1) / epb;
-    const unsigned blocks = (unsigned)(need < 148 * 2 ? need : 148 * 2);
-    kern<<<blocks, epb * group, smem, stream>>>(p, ne, batch, coords, conn, u, state, alpha_n, want_tangent, force,
-                                                tangent, energy, trial, alpha_out, yield, iterations, code,
-                                                first_failure, s.fallback, s.counts + 1);
-    return (int)cudaGetLastError();
-  };
+  return 0;
+}
+
+// The elements handed on, by a list kernel that starts each again with
+// `record` bytes of shared memory an element (one block of it per SM).
+template <class K, class... A>
+int run_list(K kern, int64_t ne, int group, size_t record, size_t* raised, cudaStream_t stream, const A&... args) {
+  const int epb = group == 8 ? 16 : 8;
+  const size_t smem = record * epb;
+  const int bad = raise_smem(kern, smem, raised);
+  if (bad) return bad;
+  const int64_t need = (ne + epb - 1) / epb;
+  kern<<<(unsigned)(need < 148 * 2 ? need : 148 * 2), epb * group, smem, stream>>>(args...);
+  return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+int launch_elements_tile(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
+                         const double* state, const double* alpha_n, int want_tangent, double* force,
+                         double* tangent, double* energy, double* trial, double* alpha_out, uint8_t* yield,
+                         int32_t* iterations, int32_t* code, int32_t* first_failure, bool batch,
+                         const TileScratch& s, int elements_per_block, cudaStream_t stream) {
+  if (ne <= 0) return 0;
+  const TileArgs a{ne, coords, conn, u, state, alpha_n, force, tangent, energy, trial, alpha_out, yield, iterations,
+                   code, first_failure, want_tangent, batch ? 1 : 0, 0, 0, 0, 0};
+  const int rc = run_tiles(p, a, s, elements_per_block, stream,
+                           [&](const TileArgs& at) { return launch_condense(p, at, s, stream); });
+  if (rc) return rc;
   static size_t raised[2][64] = {};
-  if (p.nq <= 8) return list(element_list_kernel<8>, 8, 16, sizeof(ElemShared<8>), raised[0]);
-  return list(element_list_kernel<32>, 32, 8, sizeof(ElemShared<32>), raised[1]);
+  if (p.nq <= 8)
+    return run_list(element_list_kernel<8>, ne, 8, sizeof(ElemShared<8>), raised[0], stream, p, ne, batch, coords,
+                    conn, u, state, alpha_n, want_tangent, force, tangent, energy, trial, alpha_out, yield,
+                    iterations, code, first_failure, s.fallback, s.counts + 1);
+  return run_list(element_list_kernel<32>, ne, 32, sizeof(ElemShared<32>), raised[1], stream, p, ne, batch, coords,
+                  conn, u, state, alpha_n, want_tangent, force, tangent, energy, trial, alpha_out, yield, iterations,
+                  code, first_failure, s.fallback, s.counts + 1);
+}
+
+int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
+               const double* state, const double* alpha_n, const double* lambda, double* energy, double* trial,
+               double* alpha_out, uint8_t* yield, int32_t* iterations, int32_t* code, int32_t* first_failure,
+               double* out, const TileScratch& s, int elements_per_block, cudaStream_t stream) {
+  if (ne <= 0) return 0;
+  const TileArgs a{ne, coords, conn, u, state, alpha_n, nullptr, nullptr, energy, trial, alpha_out, yield, iterations,
+                   code, first_failure, 0, 0, 0, 0, 0, 0};
+  const int rc = run_tiles(p, a, s, elements_per_block, stream,
+                           [&](const TileArgs& at) { return launch_vjp_tile(p, at, s, lambda, out, stream); });
+  if (rc) return rc;
+  static size_t raised[2][64] = {};
+  if (p.nq <= 8)
+    return run_list(vjp_kernel<8>, ne, 8, sizeof(ElemShared<8>), raised[0], stream, p, ne, coords, conn, u, state,
+                    alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
+  return run_list(vjp_kernel<32>, ne, 32, sizeof(ElemShared<32>), raised[1], stream, p, ne, coords, conn, u, state,
+                  alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
 }
 
 size_t element_smem_bytes(int group) {

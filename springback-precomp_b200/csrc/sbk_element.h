@@ -40,11 +40,12 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
 // The shape derivative: per element lambda . d f*/d X (24, node-major) into
 // out, at u with the committed points (state) and modes (alpha_n) as the
 // history and lambda a global DOF vector; the local iteration runs again to
-// the modes' equilibrium (its trial state and yield flags into trial and
-// yield). Mesh mode only.
+// the modes' equilibrium (its energies, trial state, modes, flags and counts
+// into the buffers given). Mesh mode only.
 int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
-               const double* state, const double* alpha_n, const double* lambda, double* trial, uint8_t* yield,
-               int32_t* code, int32_t* first_failure, double* out, cudaStream_t stream);
+               const double* state, const double* alpha_n, const double* lambda, double* energy, double* trial,
+               double* alpha_out, uint8_t* yield, int32_t* iterations, int32_t* code, int32_t* first_failure,
+               double* out, const TileScratch& s, int elements_per_block, cudaStream_t stream);
 // Stress recovery of ne mesh elements at u from the committed points and
 // modes: 28 doubles per element into out (see stress_kernel); the returns
 // write their (reproduced) states into scratch (the state layout).

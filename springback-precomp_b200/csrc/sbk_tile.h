@@ -78,6 +78,9 @@ inline int64_t tile_chunk(int nq) { return (int64_t)((size_t(1) << 30) / (cond_r
 // The condensation of the launch's elements whose code is 0: force and,
 // wanted, K*.
 int launch_condense(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream);
+// Their shape derivatives (24 an element) into out (sbk_vjp.cu).
+int launch_vjp_tile(const Params& p, const TileArgs& a, const TileScratch& s, const double* lambda, double* out,
+                    cudaStream_t stream);
 
 // Bytes of one allocation that tile_scratch_carve splits, for ne elements of
 // nq points.
