@@ -297,7 +297,7 @@ int sbk_system_add_node_blocks(sbk_system* sys, int32_t n, const int32_t* nodes_
  * largest strain component, the smallest det F, the averages of the
  * Kirchhoff stress (6) and of the log strain (6, tensor components; zero
  * unless logarithmic). SBK_ERR_SOLVER names the lowest failing element.
- * The trial state of the last evaluate is overwritten. */
+ * The trial state of the last evaluate can no longer be committed. */
 int sbk_system_stress(sbk_system* sys, const double* u_dev, double* out_dev);
 
 /* stiffness_gross(K, u, free) (NonlinearSystem.hpp:49-67): the norm over the

@@ -945,11 +945,9 @@ int sbk_system_stress(sbk_system* sys, const double* u_dev, double* out_dev) {
   if (!sys || !u_dev || !out_dev) return fail(SBK_ERR_ARGUMENT, "null argument");
   cudaStream_t st = sys->stream;
   SBK_CUDA(cudaMemsetAsync(sys->first_fail, 0x7f, sizeof(int32_t), st));
-  // The returns reproduce the committed states into the trial buffer, which
-  // the last evaluate's trial state no longer occupies after a commit.
   sys->has_trial = false;
-  int rc = sbk::launch_stress(sys->p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c, sys->trial,
-                              out_dev, sys->code, sys->first_fail, st);
+  int rc = sbk::launch_stress(sys->p, sys->ne, sys->coords, sys->conn, u_dev, sys->committed, sys->alpha_c, out_dev,
+                              sys->code, sys->first_fail, st);
   if (rc) return fail(SBK_ERR_CUDA, std::string("stress kernel: ") + cudaGetErrorString((cudaError_t)rc));
   int32_t first = 0;
   SBK_CUDA(cudaMemcpyAsync(&first, sys->first_fail, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

@@ -47,11 +47,10 @@ int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t*
                double* alpha_out, uint8_t* yield, int32_t* iterations, int32_t* code, int32_t* first_failure,
                double* out, const TileScratch& s, int elements_per_block, cudaStream_t stream);
 // Stress recovery of ne mesh elements at u from the committed points and
-// modes: 28 doubles per element into out (see stress_kernel); the returns
-// write their (reproduced) states into scratch (the state layout).
+// modes: 28 doubles per element into out (sbk_stress.cu).
 int launch_stress(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
-                  const double* state, const double* alpha_n, double* scratch, double* out, int32_t* code,
-                  int32_t* first_failure, cudaStream_t stream);
+                  const double* state, const double* alpha_n, double* out, int32_t* code, int32_t* first_failure,
+                  cudaStream_t stream);
 
 // The gather maps of the assembly (built once on the host).
 struct GatherMaps {

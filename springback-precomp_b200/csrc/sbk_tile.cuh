@@ -109,50 +109,22 @@ struct Tile {
     TileElement& E = el[k];
     const int pt = k * nq + q;
     const double* X = rec + 48 * k;  // staged over the record's first fields
-    const double* U = X + 24;
-    double j0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, jq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, du[9];
-    double uq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const double xi = p.qp[q][0], eta = p.qp[q][1], zeta = p.qp[q][2];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const double sx = ((n + 1) >> 1) & 1 ? 1.0 : -1.0, sy = (n >> 1) & 1 ? 1.0 : -1.0, sz = n >> 2 ? 1.0 : -1.0;
-      const double fx = 1.0 + xi * sx, fy = 1.0 + eta * sy, fz = 1.0 + zeta * sz;
-      const double dn[3] = {0.125 * sx * fy * fz, 0.125 * sy * fx * fz, 0.125 * sz * fx * fy};
-      const double d0[3] = {0.125 * sx, 0.125 * sy, 0.125 * sz};
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const double x = X[3 * n + i], u = U[3 * n + i];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          j0[i * 3 + c] += x * d0[c];
-          jq[i * 3 + c] += x * dn[c];
-          uq[i * 3 + c] += u * dn[c];
-        }
-      }
-    }
-    const double det0 = det3(j0), det = det3(jq);
-    if (!(det0 > 0.0) || !(det > 0.0)) {
+    PointGeometry G;
+    if (!point_geometry(p, q, X, X + 24, G)) {
       atomicMin(&E.fail, SBK_EL_MESH_INVERTED);
       return;
     }
-    double ji[9];
-    if (q == 0) {
-      inv3(j0, ji);
+    if (q == 0)
 #pragma unroll
-      for (int i = 0; i < 9; ++i) E.jinv0[i] = ji[i];
-    }
-    inv3(jq, ji);
-    rec[kRecW * np + pt] = p.qp[q][3] * det;
+      for (int i = 0; i < 9; ++i) E.jinv0[i] = G.j0i[i];
+    rec[kRecW * np + pt] = G.w;
     double* g = geo + pt;
 #pragma unroll
-    for (int i = 0; i < 9; ++i) g[i * np] = ji[i];
-    g[9 * np] = det0 / det;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) du[i * 3 + j] = uq[i * 3] * ji[j] + uq[i * 3 + 1] * ji[3 + j] + uq[i * 3 + 2] * ji[6 + j];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g[(10 + i) * np] = du[i];
+    for (int i = 0; i < 9; ++i) {
+      g[i * np] = G.ji[i];
+      g[(10 + i) * np] = G.du[i];
+    }
+    g[9 * np] = G.ratio;
   }
 
   // Kinematics, log strain and trial state of a point at its element's trial
@@ -180,45 +152,21 @@ struct Tile {
 #pragma unroll
     for (int i = 0; i < 9; ++i) hmax = fmax(hmax, fabs(h[i]));
     double strain[6];
-    int code = 0;
-    if (p.kinematics == SBK_SMALL_STRAIN) {
-      strain[0] = h[0], strain[1] = h[4], strain[2] = h[8];
-      strain[3] = h[1] + h[3], strain[4] = h[5] + h[7], strain[5] = h[6] + h[2];
-    } else {
-      double E2[6];  // twice the Green-Lagrange strain
+    LogKin L;
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const int i = c < 3 ? c : c - 3, j = c < 3 ? c : (c - 2) % 3;
-        E2[c] = h[i * 3 + j] + h[j * 3 + i] + h[i] * h[j] + h[3 + i] * h[3 + j] + h[6 + i] * h[6 + j];
-      }
-#pragma unroll
-      for (int c = 0; c < 6; ++c) strain[c] = c < 3 ? 0.5 * E2[c] : E2[c];
-      if (p.kinematics == SBK_FINITE_LOGARITHMIC) {
-        const double F[9] = {h[0] + 1.0, h[1], h[2], h[3], h[4] + 1.0, h[5], h[6], h[7], h[8] + 1.0};
-        if (!(det3(F) > 0.0)) {
-          code = SBK_EL_INVERTED_POINT;
-        } else {
-          LogKin L;
-#pragma unroll
-          for (int i = 0; i < 9; ++i) L.q[i] = first ? (i % 4 == 0 ? 1.0 : 0.0) : r.get(kRecL + i);
-          double green[6];
-#pragma unroll
-          for (int c = 0; c < 6; ++c) green[c] = strain[c];
-          code = spectral_log(green, L, strain);
-          if (!code) {
-#pragma unroll
-            for (int i = 0; i < 9; ++i) r.put(kRecL + i, L.q[i]);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) r.put(kRecL + 9 + i, L.mu[i]);
-#pragma unroll
-            for (int i = 0; i < 6; ++i) r.put(kRecL + 12 + i, L.first[i]);
-          }
-        }
-      }
-    }
+    for (int i = 0; i < 9; ++i) L.q[i] = first ? (i % 4 == 0 ? 1.0 : 0.0) : r.get(kRecL + i);
+    const int code = point_strain(p, h, L, strain);
     if (code) {
       atomicMin(&E.fail, (1 << 16) | (q << 8) | code);
       return false;
+    }
+    if (p.kinematics == SBK_FINITE_LOGARITHMIC) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) r.put(kRecL + i, L.q[i]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) r.put(kRecL + 9 + i, L.mu[i]);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) r.put(kRecL + 12 + i, L.first[i]);
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) r.put(kRecH + i, h[i]);

@@ -10,6 +10,7 @@
 // up to four (their count read from the parameters).
 #pragma once
 
+#include "sbk_element_math.cuh"
 #include "sbk_material.cuh"
 
 namespace sbk {
@@ -168,6 +169,70 @@ __device__ __forceinline__ int spectral_log(const double green[6], LogKin& L, do
 #pragma unroll
   for (int i = 3; i < 6; ++i) elog[i] *= 2.0;
   return 0;
+}
+
+// Reference geometry of a point (set_up, IncompatibleModes.cpp:134-192) from its
+// element's staged coordinates and displacements X, U (24 each): J^-1, w det
+// J, det0 / det, J0^-1 and U G^T. False for an element inverted at rest.
+struct PointGeometry {
+  double ji[9], j0i[9], du[9], w, ratio;
+};
+__device__ __forceinline__ bool point_geometry(const Params& p, int q, const double* X, const double* U,
+                                               PointGeometry& G) {
+  double j0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, jq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  double uq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const double xi = p.qp[q][0], eta = p.qp[q][1], zeta = p.qp[q][2];
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    const double sx = ((n + 1) >> 1) & 1 ? 1.0 : -1.0, sy = (n >> 1) & 1 ? 1.0 : -1.0, sz = n >> 2 ? 1.0 : -1.0;
+    const double fx = 1.0 + xi * sx, fy = 1.0 + eta * sy, fz = 1.0 + zeta * sz;
+    const double dn[3] = {0.125 * sx * fy * fz, 0.125 * sy * fx * fz, 0.125 * sz * fx * fy};
+    const double d0[3] = {0.125 * sx, 0.125 * sy, 0.125 * sz};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double x = X[3 * n + i], u = U[3 * n + i];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        j0[i * 3 + c] += x * d0[c];
+        jq[i * 3 + c] += x * dn[c];
+        uq[i * 3 + c] += u * dn[c];
+      }
+    }
+  }
+  const double det0 = det3(j0), det = det3(jq);
+  if (!(det0 > 0.0) || !(det > 0.0)) return false;
+  inv3(j0, G.j0i);
+  inv3(jq, G.ji);
+  G.w = p.qp[q][3] * det;
+  G.ratio = det0 / det;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      G.du[i * 3 + j] = uq[i * 3] * G.ji[j] + uq[i * 3 + 1] * G.ji[3 + j] + uq[i * 3 + 2] * G.ji[6 + j];
+  return true;
+}
+
+// The strain the return takes at the displacement gradient h, with L (from the
+// axes it holds) under logarithmic kinematics. 0 or the point's failure.
+__device__ __forceinline__ int point_strain(const Params& p, const double h[9], LogKin& L, double strain[6]) {
+  if (p.kinematics == SBK_SMALL_STRAIN) {
+    strain[0] = h[0], strain[1] = h[4], strain[2] = h[8];
+    strain[3] = h[1] + h[3], strain[4] = h[5] + h[7], strain[5] = h[6] + h[2];
+    return 0;
+  }
+  double green[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const int i = c < 3 ? c : c - 3, j = c < 3 ? c : (c - 2) % 3;
+    const double e2 = h[i * 3 + j] + h[j * 3 + i] + h[i] * h[j] + h[3 + i] * h[3 + j] + h[6 + i] * h[6 + j];
+    green[c] = c < 3 ? 0.5 * e2 : e2;
+    strain[c] = green[c];
+  }
+  if (p.kinematics != SBK_FINITE_LOGARITHMIC) return 0;
+  const double F[9] = {h[0] + 1.0, h[1], h[2], h[3], h[4] + 1.0, h[5], h[6], h[7], h[8] + 1.0};
+  if (!(det3(F) > 0.0)) return SBK_EL_INVERTED_POINT;
+  return spectral_log(green, L, strain);
 }
 
 // second(k, j, i), mu_k <= mu_j <= mu_i: the second divided difference of ln
@@ -556,8 +621,8 @@ __device__ __forceinline__ void return_tangent(const Params& p, const ReturnPoin
 // is the smaller one; if that does not converge the return runs again from
 // the trial state. One loop evaluates every candidate - start, Newton trial,
 // polishing step - so that the equations and their factors are in the code
-// once.
-template <int NT>
+// once. TANGENT = false: the stress alone.
+template <int NT, bool TANGENT = true>
 __device__ __forceinline__ int return_general(const Params& p, const PointTrial<NT>& P, bool window, bool warm,
                                               const PointRecord& rec, int fS, int fM, int fW) {
   ReturnTrial<NT> T;
@@ -663,7 +728,7 @@ __device__ __forceinline__ int return_general(const Params& p, const PointTrial<
     rec.put(fS + k, P.s[k] - 2.0 * p.G * n.dl * m[k] + (k < 3 ? p.K * P.vol : 0.0));
   }
   if (!window) rec.put(fW + 6, n.dl);
-  return_tangent(p, n, r, rec, fM);
+  if (TANGENT) return_tangent(p, n, r, rec, fM);
   return 0;
 }
 
@@ -686,6 +751,7 @@ __device__ __forceinline__ void return_window_radial(const Params& p, const Poin
 
 // The plastic J2 return (radial_return): stress and tangent into the record,
 // the flow direction and dgamma into its warm fields.
+template <bool TANGENT = true>
 __device__ __forceinline__ int return_radial(const Params& p, const PointTrial<-1>& T, const PointRecord& rec, int fS,
                                              int fM, int fW) {
   const double g = p.G, k = p.K, hk = p.Hkin;
@@ -722,7 +788,7 @@ __device__ __forceinline__ int return_radial(const Params& p, const PointTrial<-
     rec.put(fS + i, T.s[i] - 2.0 * g * dgamma * n[i] + (i < 3 ? k * T.vol : 0.0));
     rec.put(fW + i, n[i]);
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
+    for (int j = 0; j < (TANGENT ? 6 : 0); ++j) {
       const double el = i < 3 ? (j < 3 ? k - 2.0 * g * theta / 3.0 : 0.0) + (i == j ? 2.0 * g * theta : 0.0)
                               : (i == j ? g * theta : 0.0);
       rec.put(fM + i * 6 + j, el - 2.0 * g * theta_bar * (n[i] * n[j]));

@@ -422,7 +422,8 @@ class NonlinearSystem:
         """elastoplastic_stress of every element at u from the committed
         points and modes (IncompatibleModes.cpp:602-664), the step-end stress
         recovery of the forming driver (Forming.cpp:1266-1281): call after
-        commit(). Overwrites the trial state of the last evaluate."""
+        commit(). The trial state of the last evaluate can no longer be
+        committed."""
         u = u.to(torch.float64).contiguous()
         if u.numel() != self.num_dofs:
             raise ValueError(f"u has {u.numel()} values, the system {self.num_dofs} DOFs")
