@@ -448,10 +448,10 @@ void free_system(sbk_system* s) {
 
 std::atomic<int> g_local_mode{SBK_LOCAL_PHASES};
 
-// The tile kernel's scratch of a system whose element takes it (allocated
-// once, outside any stream capture).
+// The tile kernels' scratch of a system (allocated once, outside any stream
+// capture).
 int ensure_tile(sbk_system* s) {
-  if (s->tile_mem || !sbk::tile_applies(s->p)) return SBK_OK;
+  if (s->tile_mem) return SBK_OK;
   cudaError_t e = cudaMalloc(&s->tile_mem, sbk::tile_scratch_bytes(s->ne, s->p.nq));
   if (e != cudaSuccess) {
     s->tile_mem = nullptr;
@@ -461,9 +461,10 @@ int ensure_tile(sbk_system* s) {
   return SBK_OK;
 }
 
-// Whether K1 of the system runs as the tile kernel.
+// Whether the system's elements run in tiles: the standard Hex8 always, the
+// incompatible-mode one unless the single kernel is asked for.
 bool uses_tiles(const sbk_system* sys) {
-  return sys->local_mode == SBK_LOCAL_PHASES && sys->tile_mem && sbk::tile_applies(sys->p);
+  return sys->tile_mem && (sys->p.element == 1 || sys->local_mode == SBK_LOCAL_PHASES);
 }
 
 // Whether the element schedule runs after an evaluation: for the single
@@ -545,7 +546,7 @@ int sbk_element_batch(const sbk_material* material, const sbk_rule* rule, int ki
     return fail(SBK_ERR_ARGUMENT, "null device buffer");
   if (ne * p.nq > 0x7fffffffLL) return fail(SBK_ERR_UNSUPPORTED, "too many points for one batch");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (g_local_mode.load() == SBK_LOCAL_PHASES && sbk::tile_applies(p)) {
+  if (g_local_mode.load() == SBK_LOCAL_PHASES) {
     // The tile kernel's scratch, stream-ordered on the caller's stream.
     void* mem = nullptr;
     SBK_CUDA(cudaMallocAsync(&mem, sbk::tile_scratch_bytes(ne, p.nq), s));
@@ -639,7 +640,7 @@ int sbk_system_create(const sbk_mesh* mesh, const sbk_material* material, const 
   TRY(dalloc(&s->scalars, 4));
   TRY(dalloc(&s->missing, 1));
   s->local_mode = g_local_mode.load();
-  TRY(ensure_tile(s));
+  if (s->local_mode == SBK_LOCAL_PHASES) TRY(ensure_tile(s));
 #undef TRY
   // Virgin points and zero modes (initialise_history).
   cudaMemset(s->committed, 0, state_size * sizeof(double));
@@ -691,11 +692,7 @@ int sbk_system_set_element(sbk_system* sys, int element, int mean_dilatation) {
                         ? 1
                         : 0;
   sys->order_valid = false;
-  if (!sbk::tile_applies(sys->p) && sys->tile_mem) {
-    cudaFree(sys->tile_mem);
-    sys->tile_mem = nullptr;
-  }
-  return sys->local_mode == SBK_LOCAL_PHASES ? ensure_tile(sys) : SBK_OK;
+  return sys->p.element == 1 || sys->local_mode == SBK_LOCAL_PHASES ? ensure_tile(sys) : SBK_OK;
 }
 
 int sbk_system_set_frozen(sbk_system* sys, int frozen) {

@@ -28,10 +28,9 @@ int launch_elements(const Params& p, int64_t ne, const double* coords, const int
                     const int32_t* order, cudaStream_t stream);
 size_t element_smem_bytes(int group);
 
-// K1 of the incompatible-mode Hex8 by the tile kernel (sbk_tile.cuh; mesh or
-// batch mode, as launch_elements), every rule; no host synchronisation, so
-// it can be captured in a CUDA graph.
-bool tile_applies(const Params& p);
+// K1 by tiles (sbk_tile.cuh; mesh or batch mode, as launch_elements), every
+// rule, and the standard Hex8 (sbk_standard.cu; mesh mode); no host
+// synchronisation, so it can be captured in a CUDA graph.
 int launch_elements_tile(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
                          const double* state, const double* alpha_n, int want_tangent, double* force,
                          double* tangent, double* energy, double* trial, double* alpha_out, uint8_t* yield,

@@ -23,7 +23,7 @@ struct TileScratch {
   int32_t* counts;    // [0] the next tile, [1] elements handed on
   int32_t* fallback;  // ne
   double* geo;        // blocks x kTileGeo x points of a tile
-  double* cond;       // tile_chunk x cond_record: the converged elements' records
+  double* cond;       // tile_chunk x tile_record: the elements' records
 };
 
 // Where an evaluation reads and writes (launch_elements' arguments).
@@ -71,9 +71,17 @@ constexpr int kCondPerm = 108; // 16 row + column of each pivot, 9
 constexpr int kCondElement = 118;
 __host__ __device__ inline size_t cond_record(int nq) { return (size_t)kCondPoint * nq + kCondElement; }
 
+// A standard Hex8's: per point the fields above, then the mean dilatation's: P^T
+// T 6, P^T C m / 3 6, P^T C^T m / 3 6, P^T m 6, m.C m / 9, tr T / 3.
+constexpr int kStdSt = 62, kStdU1 = 68, kStdU2 = 74, kStdPv = 80, kStdMcm = 86, kStdTr = 87, kStdPoint = 88;
+// Doubles an element of the scratch takes, for either element.
+__host__ __device__ inline size_t tile_record(int nq) {
+  return cond_record(nq) > (size_t)kStdPoint * nq ? cond_record(nq) : (size_t)kStdPoint * nq;
+}
+
 // Elements of one launch: what 1 GiB of records holds (a mesh of more takes
 // several launches, so that the scratch does not grow with it).
-inline int64_t tile_chunk(int nq) { return (int64_t)((size_t(1) << 30) / (cond_record(nq) * sizeof(double))); }
+inline int64_t tile_chunk(int nq) { return (int64_t)((size_t(1) << 30) / (tile_record(nq) * sizeof(double))); }
 
 // The condensation of the launch's elements whose code is 0: force and,
 // wanted, K*.
@@ -81,6 +89,9 @@ int launch_condense(const Params& p, const TileArgs& a, const TileScratch& s, cu
 // Their shape derivatives (24 an element) into out (sbk_vjp.cu).
 int launch_vjp_tile(const Params& p, const TileArgs& a, const TileScratch& s, const double* lambda, double* out,
                     cudaStream_t stream);
+
+// The standard Hex8 over the launch's elements (sbk_standard.cu).
+int launch_standard(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream);
 
 // Bytes of one allocation that tile_scratch_carve splits, for ne elements of
 // nq points.
