@@ -488,8 +488,9 @@ int sbk_partition_add_to(sbk_partition* part, double* full_dev, const double* v_
 /* PartitionedFactor::factorize (Forming.cpp:100-160) of the free-free block
  * of values_dev (the full tangent, device), where the reference takes
  * CHOLMOD's supernodal Cholesky, then LDL^T, then LU (UMFPACK):
- *   symmetric: a sparse Cholesky on the device (cuSOLVER), its pattern
- *     analysed on the first call;
+ *   symmetric: a multifrontal sparse Cholesky on the device, its pattern
+ *     analysed on the first call (cuSOLVER's level-scheduled one where the
+ *     dense fronts would take over six tenths of the device's free memory);
  *   not symmetric, or a Cholesky that meets a non-positive pivot or whose
  *     correction's backward error exceeds 1e-10: a dense LU with partial
  *     pivoting on the device while the block has at most the dense limit of

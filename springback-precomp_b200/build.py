@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libsbk.so")
 SOURCES = ["sbk_element.cu", "sbk_assembly.cu", "sbk_contact.cu", "sbk_capi.cu", "sbk_schedule.cu", "sbk_noalloc.cu",
            "sbk_pattern.cu", "sbk_tile_j2.cu", "sbk_tile_general0.cu", "sbk_tile_general1.cu", "sbk_tile_general2.cu",
            "sbk_tile_general4.cu", "sbk_condense.cu", "sbk_vjp.cu", "sbk_stress.cu",
-           "sbk_standard.cu",
+           "sbk_standard.cu", "sbk_multifrontal.cu",
            "sbk_partition.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -8,21 +8,22 @@
 // column are free, in the full pattern's order (ff_src: the full index of
 // each block entry, the inverse of the reference's positions_ map), so that
 // assemble is one gather. The factorisation takes B = K_ff(p, p) in CSR
-// with p a METIS nested-dissection order; fac_src maps every entry of B
+// with p a METIS nested-dissection order of the nodes, each node's free DOFs
+// together, in the postorder of its elimination tree; fac_src maps every entry of B
 // straight to its full index (transposition and permutation composed on
 // the host at build time), so that factorize also reads the full tangent
 // once, with no intermediate copy of the block.
 //
-// A symmetric block takes a sparse Cholesky. A non-symmetric one (Chaboche
-// backstresses with recovery, the exact friction tangent), or one whose
+// A symmetric block takes a multifrontal Cholesky (sbk_multifrontal.cu; the
+// library's level-scheduled one where its fronts do not fit the device). A
+// non-symmetric one (Chaboche backstresses with recovery, the exact friction tangent), or one whose
 // Cholesky fails, takes a dense LU with partial pivoting while it has at most
 // kDenseMax rows (n^2 doubles: 3.2 GB at the bound); a larger one takes
 // restarted GMRES preconditioned by the Cholesky of its symmetric part, and
 // a sparse QR when that stalls or the symmetric part is not positive
-// definite. The factorisations (cuSOLVER's device sparse Cholesky, dense LU
-// and sparse QR) are library code; the gathers, the permutations, the
-// densification, the Krylov iteration and the backward-error check are this
-// file's.
+// definite. The dense LU and the sparse QR are cuSOLVER's; the gathers, the
+// permutations, the densification, the Krylov iteration and the
+// backward-error check are this file's.
 #define DISABLE_CUSOLVER_DEPRECATED
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
@@ -33,11 +34,13 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <string>
 #include <utility>
 #include <vector>
 
 #include "sbk.h"
+#include "sbk_multifrontal.h"
 
 namespace sbk {
 int set_error(int code, const std::string& what);
@@ -194,15 +197,26 @@ __global__ void max_abs_kernel(const double* __restrict__ a, int64_t n, unsigned
 __global__ void backward_error_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                                       const double* __restrict__ val, const double* __restrict__ x,
                                       const double* __restrict__ b, int32_t n, unsigned long long* out) {
+  // Eight lanes a row: its entries are read together.
   double rmax = 0.0, smax = 0.0;
   int bad = 0;
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double r = -b[i], s = fabs(b[i]);
-    for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-      const double t = val[k] * x[col[k]];
-      r += t;
-      s += fabs(t);
+  const int lane = threadIdx.x & 7;
+  for (int32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 2; i0 < n; i0 += gridDim.x * blockDim.x >> 3) {
+    const int32_t i = i0 + ((threadIdx.x & 31) >> 3);
+    double r = 0.0, s = 0.0;
+    if (i < n)
+      for (int32_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 8) {
+        const double t = val[k] * x[col[k]];
+        r += t;
+        s += fabs(t);
+      }
+    for (int o = 4; o > 0; o >>= 1) {
+      r += __shfl_xor_sync(0xffffffffu, r, o);
+      s += __shfl_xor_sync(0xffffffffu, s, o);
     }
+    if (i >= n) continue;
+    r -= b[i];
+    s += fabs(b[i]);
     if (!isfinite(r) || !isfinite(s)) {
       bad = 1;
     } else {
@@ -266,6 +280,12 @@ struct sbk_partition {
   // cuSOLVER
   cusolverSpHandle_t handle = nullptr;
   cusparseMatDescr_t descr = nullptr;
+  // the Cholesky: multifrontal, its analysis made with the first
+  // factorisation that takes it, or the library's
+  sbk::FrontOrder order;
+  std::vector<int32_t> host_rowptr, host_col;
+  sbk::Multifrontal* fronts = nullptr;
+  int32_t* pivot = nullptr;
   csrcholInfo_t chol = nullptr;
   void* chol_work = nullptr;
   bool analysed = false;
@@ -288,6 +308,8 @@ struct sbk_partition {
       if (p) cudaFree(p);
     for (void* p : {(void*)lu, (void*)ipiv, (void*)lu_info, (void*)lu_work})
       if (p) cudaFree(p);
+    if (pivot) cudaFree(pivot);
+    delete fronts;
     if (dense) cusolverDnDestroy(dense);
     if (chol) cusolverSpDestroyCsrcholInfo(chol);
     if (descr) cusparseDestroyMatDescr(descr);
@@ -336,20 +358,52 @@ int build_partition(sbk_partition* P, const std::vector<int32_t>& outer, const s
       tr[(size_t)t] = (int32_t)(it - ff_inner.begin());
     }
   }
-  // Fill-reducing order: the block's pattern read as CSR is its own (it is
-  // symmetric).
-  std::vector<int32_t> p((size_t)nf), pinv((size_t)nf);
-  PSOLVER(cusolverSpXcsrmetisndHost(P->handle, nf, (int)m, P->descr, ff_outer.data(), ff_inner.data(), nullptr,
-                                    p.data()));
+  // Fill-reducing order of the nodes (three DOFs each): their graph has a
+  // ninth of the block's entries.
+  std::vector<std::vector<int32_t>> members;
+  std::vector<int32_t> group((size_t)nf);
+  for (int32_t i = 0; i < nf; ++i) {
+    if (i == 0 || free[(size_t)i] / 3 != free[(size_t)i - 1] / 3) members.emplace_back();
+    members.back().push_back(i);
+    group[(size_t)i] = (int32_t)members.size() - 1;
+  }
+  const int32_t ng = (int32_t)members.size();
+  std::vector<int32_t> gptr((size_t)ng + 1, 0), gadj, dptr((size_t)ng + 1, 0), dadj, seen((size_t)ng, -1), fill((size_t)ng);
+  for (int32_t g = 0; g < ng; ++g) {
+    const size_t from = dadj.size();
+    seen[(size_t)g] = g;
+    dadj.push_back(g);
+    for (int32_t c : members[(size_t)g])
+      for (int32_t t = ff_outer[(size_t)c]; t < ff_outer[(size_t)c + 1]; ++t) {
+        const int32_t h = group[(size_t)ff_inner[(size_t)t]];
+        if (seen[(size_t)h] != g) {
+          seen[(size_t)h] = g;
+          dadj.push_back(h);
+          gadj.push_back(h);
+        }
+      }
+    std::sort(dadj.begin() + (ptrdiff_t)from, dadj.end());
+    std::sort(gadj.begin() + gptr[(size_t)g], gadj.end());
+    dptr[(size_t)g + 1] = (int32_t)dadj.size();
+    gptr[(size_t)g + 1] = (int32_t)gadj.size();
+  }
+  if (ng > 2) {
+    PSOLVER(cusolverSpXcsrmetisndHost(P->handle, ng, (int)dadj.size(), P->descr, dptr.data(), dadj.data(), nullptr,
+                                      fill.data()));
+  } else {
+    for (int32_t g = 0; g < ng; ++g) fill[(size_t)g] = g;
+  }
   {
-    std::vector<char> seen((size_t)nf, 0);
-    for (int32_t i = 0; i < nf; ++i) {
-      if (p[(size_t)i] < 0 || p[(size_t)i] >= nf || seen[(size_t)p[(size_t)i]])
-        return pfail(SBK_ERR_CUDA, "the fill-reducing order is not a permutation");
-      seen[(size_t)p[(size_t)i]] = 1;
-      pinv[(size_t)p[(size_t)i]] = i;
+    std::fill(seen.begin(), seen.end(), 0);
+    for (int32_t g : fill) {
+      if (g < 0 || g >= ng || seen[(size_t)g]) return pfail(SBK_ERR_CUDA, "the fill-reducing order is not a permutation");
+      seen[(size_t)g] = 1;
     }
   }
+  sbk::front_order(fill, members, gptr, gadj, P->order);
+  const std::vector<int32_t>& p = P->order.perm;
+  std::vector<int32_t> pinv((size_t)nf);
+  for (int32_t i = 0; i < nf; ++i) pinv[(size_t)p[(size_t)i]] = i;
   // B = K_ff(p, p) in CSR. Row i of B is the block's row r = p[i]; its
   // entries (r, q) sit, in the CSC block, in column q at row r: the mirror
   // tr[t] of entry t = (q, r) of column r.
@@ -391,6 +445,9 @@ int build_partition(sbk_partition* P, const std::vector<int32_t>& outer, const s
   if (int rc = alloc(&P->rhs, nf)) return rc;
   if (int rc = alloc(&P->sol, nf)) return rc;
   if (int rc = alloc(&P->check, 4)) return rc;
+  if (int rc = alloc(&P->pivot, 1)) return rc;
+  P->host_rowptr = std::move(rowptr);
+  P->host_col = std::move(col);
   return SBK_OK;
 }
 
@@ -398,7 +455,7 @@ int build_partition(sbk_partition* P, const std::vector<int32_t>& outer, const s
 // + |rhs|), or infinity when a row's sums are not finite.
 int backward_error(sbk_partition* P, double* omega) {
   PCUDA(cudaMemsetAsync(P->check, 0, 3 * sizeof(unsigned long long), P->stream));
-  backward_error_kernel<<<grid_for(P->nf), kThreads, 0, P->stream>>>(P->fac_rowptr, P->fac_col, P->fac_val, P->sol,
+  backward_error_kernel<<<grid_for(8 * (int64_t)P->nf), kThreads, 0, P->stream>>>(P->fac_rowptr, P->fac_col, P->fac_val, P->sol,
                                                                      P->rhs, P->nf, P->check);
   PCUDA(cudaGetLastError());
   unsigned long long h[3];
@@ -423,7 +480,63 @@ int solve_qr(sbk_partition* P) {
   return SBK_OK;
 }
 
+// The Cholesky's analysis, with the first factorisation that takes it. The
+// multifrontal one may take six tenths of the device's free memory.
+int chol_analyse(sbk_partition* P, const double* values) {
+  if (P->analysed) return SBK_OK;
+  size_t room = 0, total = 0;
+  PCUDA(cudaMemGetInfo(&room, &total));
+  P->fronts = new sbk::Multifrontal;
+  cudaError_t err = cudaErrorMemoryAllocation;
+  try {
+    err = P->fronts->build(P->order, P->host_rowptr, P->host_col, room / 10 * 6);
+  } catch (const std::bad_alloc&) {  // the host's tables
+  }
+  if (err != cudaSuccess) {
+    delete P->fronts;
+    P->fronts = nullptr;
+    cudaGetLastError();
+    if (err != cudaErrorMemoryAllocation)
+      return pfail(SBK_ERR_CUDA, std::string("the Cholesky's analysis: ") + cudaGetErrorString(err));
+    PSOLVER(cusolverSpCreateCsrcholInfo(&P->chol));
+    PSOLVER(cusolverSpXcsrcholAnalysis(P->handle, P->nf, (int)P->nnz_ff, P->descr, P->fac_rowptr, P->fac_col,
+                                       P->chol));
+    size_t internal = 0, work = 0;
+    PSOLVER(cusolverSpDcsrcholBufferInfo(P->handle, P->nf, (int)P->nnz_ff, P->descr, values, P->fac_rowptr,
+                                         P->fac_col, P->chol, &internal, &work));
+    PCUDA(cudaMalloc(&P->chol_work, work > 0 ? work : 1));
+  }
+  P->analysed = true;
+  P->order = sbk::FrontOrder();
+  std::vector<int32_t>().swap(P->host_rowptr);
+  std::vector<int32_t>().swap(P->host_col);
+  return SBK_OK;
+}
+
+// The Cholesky of `values` in B's pattern; *definite: every pivot positive.
+int chol_factor(sbk_partition* P, const double* values, bool* definite) {
+  if (int rc = chol_analyse(P, values)) return rc;
+  if (P->fronts) {
+    PCUDA(P->fronts->factor(values, P->pivot, P->stream));
+    int32_t failed = 0;
+    PCUDA(cudaMemcpyAsync(&failed, P->pivot, sizeof(failed), cudaMemcpyDeviceToHost, P->stream));
+    PCUDA(cudaStreamSynchronize(P->stream));
+    *definite = failed == 0x7f7f7f7f;
+    return SBK_OK;
+  }
+  PSOLVER(cusolverSpDcsrcholFactor(P->handle, P->nf, (int)P->nnz_ff, P->descr, values, P->fac_rowptr, P->fac_col,
+                                   P->chol, P->chol_work));
+  int position = -1;
+  PSOLVER(cusolverSpDcsrcholZeroPivot(P->handle, P->chol, 0.0, &position));
+  *definite = position < 0;
+  return SBK_OK;
+}
+
 int chol_apply(sbk_partition* P, const double* b, double* x) {
+  if (P->fronts) {
+    PCUDA(P->fronts->solve(b, x, P->stream));
+    return SBK_OK;
+  }
   PSOLVER(cusolverSpDcsrcholSolve(P->handle, P->nf, b, x, P->chol, P->chol_work));
   return SBK_OK;
 }
@@ -709,21 +822,9 @@ int sbk_partition_factorize(sbk_partition* part, const double* values_dev, int s
       PCUDA(cudaGetLastError());
       chol_val = P->sym_val;
     }
-    if (!P->analysed) {
-      PSOLVER(cusolverSpCreateCsrcholInfo(&P->chol));
-      PSOLVER(cusolverSpXcsrcholAnalysis(P->handle, P->nf, (int)P->nnz_ff, P->descr, P->fac_rowptr, P->fac_col,
-                                         P->chol));
-      size_t internal = 0, work = 0;
-      PSOLVER(cusolverSpDcsrcholBufferInfo(P->handle, P->nf, (int)P->nnz_ff, P->descr, chol_val, P->fac_rowptr,
-                                           P->fac_col, P->chol, &internal, &work));
-      PCUDA(cudaMalloc(&P->chol_work, work > 0 ? work : 1));
-      P->analysed = true;
-    }
-    PSOLVER(cusolverSpDcsrcholFactor(P->handle, P->nf, (int)P->nnz_ff, P->descr, chol_val, P->fac_rowptr,
-                                     P->fac_col, P->chol, P->chol_work));
-    int position = -1;
-    PSOLVER(cusolverSpDcsrcholZeroPivot(P->handle, P->chol, 0.0, &position));
-    if (position < 0) {
+    bool definite = false;
+    if (int rc = chol_factor(P, chol_val, &definite)) return rc;
+    if (definite) {
       P->kind = symmetric ? SBK_FACTOR_CHOLESKY : SBK_FACTOR_GMRES;
       ++P->counts[symmetric ? kCholesky : kGmres];
     } else {

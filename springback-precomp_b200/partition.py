@@ -8,8 +8,8 @@ K_ff x = b; `restrict` and `add_to` are the driver's vector helpers
 (src/fem/NonlinearSystem.hpp:336-347). The pattern of the block, its
 fill-reducing order and the gather maps are built once per partition; every
 iteration then reads the full tangent once. The factorisations are
-cuSOLVER's device sparse Cholesky for a symmetric block; for a
-non-symmetric one (Chaboche recovery, exact friction tangent) or one that is
+a multifrontal Cholesky on the device for a symmetric block (cuSOLVER's
+where its dense fronts do not fit); for a non-symmetric one (Chaboche recovery, exact friction tangent) or one that is
 not positive definite, a dense LU on the device up to the dense limit
 (20000 rows by default), beyond it restarted GMRES preconditioned by the
 Cholesky of the symmetric part and the device sparse QR where that fails -
