@@ -357,6 +357,15 @@ int dalloc(T** ptr, size_t count) {
   return SBK_OK;
 }
 
+// Page-locked doubles that a kernel writes and the host reads after its
+// synchronisation.
+int pinned(double** ptr, size_t count) {
+  *ptr = nullptr;
+  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(ptr), count * sizeof(double), cudaHostAllocMapped);
+  if (e != cudaSuccess) return fail(SBK_ERR_CUDA, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+  return SBK_OK;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -391,6 +400,7 @@ struct sbk_system {
   double* internal = nullptr;
   double* scratch = nullptr;
   double* scalars = nullptr;
+  double* host = nullptr;  // page-locked: an evaluation's sums and lowest failing element, a missing block
   int32_t* missing = nullptr;
   int32_t* block_col = nullptr;
   int64_t* block_value = nullptr;
@@ -441,6 +451,7 @@ void free_system(sbk_system* s) {
                   s->order, s->sched, s->tile_mem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (s->host) cudaFreeHost(s->host);
   for (cudaEvent_t e : s->ev)
     if (e) cudaEventDestroy(e);
   delete s;
@@ -639,6 +650,7 @@ int sbk_system_create(const sbk_mesh* mesh, const sbk_material* material, const 
   TRY(dalloc(&s->scratch, sbk::assemble_scratch_doubles()));
   TRY(dalloc(&s->scalars, 4));
   TRY(dalloc(&s->missing, 1));
+  TRY(pinned(&s->host, 5));
   s->local_mode = g_local_mode.load();
   if (s->local_mode == SBK_LOCAL_PHASES) TRY(ensure_tile(s));
 #undef TRY
@@ -769,7 +781,7 @@ int sbk_system_evaluate(sbk_system* sys, const double* u_dev, double lambda, int
   // it, with the scalars, in a single synchronisation (its sums are then
   // discarded, as the reference discards them when it throws).
   rc = sbk::launch_assemble_forces(sys->maps(), sys->force, sys->energy_e, sys->yield, sys->p.nq, sys->internal,
-                                   sys->scratch, sys->scalars, st);
+                                   sys->scratch, sys->scalars, sys->first_fail, sys->host, st);
   if (rc) return fail(SBK_ERR_CUDA, std::string("assembly: ") + cudaGetErrorString((cudaError_t)rc));
   if (sys->timing) SBK_CUDA(cudaEventRecord(sys->ev[2], st));
   if (want_tangent) {
@@ -782,11 +794,9 @@ int sbk_system_evaluate(sbk_system* sys, const double* u_dev, double lambda, int
     if (rc) return fail(SBK_ERR_CUDA, std::string("schedule: ") + cudaGetErrorString((cudaError_t)rc));
     sys->order_valid = true;
   }
-  double sc[3];
-  int32_t first = 0;
-  SBK_CUDA(cudaMemcpyAsync(sc, sys->scalars, sizeof(sc), cudaMemcpyDeviceToHost, st));
-  SBK_CUDA(cudaMemcpyAsync(&first, sys->first_fail, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   SBK_CUDA(cudaStreamSynchronize(st));
+  const double* sc = sys->host;
+  const int32_t first = static_cast<int32_t>(sc[3]);
   if (sys->timing) {
     float ms = 0.0f;
     for (int i = 0; i < 3; ++i) {
@@ -861,7 +871,7 @@ int sbk_system_enqueue(sbk_system* sys, const double* u_dev, int want_tangent, d
   int rc = system_elements(sys, u_dev, want_tangent, st);
   if (rc) return fail(SBK_ERR_CUDA, std::string("element kernel: ") + cudaGetErrorString((cudaError_t)rc));
   rc = sbk::launch_assemble_forces(sys->maps(), sys->force, sys->energy_e, sys->yield, sys->p.nq, sys->internal,
-                                   sys->scratch, sys->scalars, st);
+                                   sys->scratch, sys->scalars, nullptr, nullptr, st);
   if (!rc && want_tangent) rc = sbk::launch_assemble_values(sys->maps(), sys->tangent, sys->values, st);
   if (!rc && schedules(sys) && sys->order_valid)
     rc = sbk::launch_schedule(sys->ne, sys->p.nq, sys->iters, sys->yield, sys->sched, sys->order, st);
@@ -927,14 +937,12 @@ int sbk_system_add_node_blocks(sbk_system* sys, int32_t n, const int32_t* nodes_
   if (!sys || (n > 0 && (!nodes_dev || !blocks_dev))) return fail(SBK_ERR_ARGUMENT, "null argument");
   if (n <= 0) return SBK_OK;
   cudaStream_t st = sys->stream;
-  SBK_CUDA(cudaMemsetAsync(sys->missing, 0, sizeof(int32_t), st));
+  sys->host[4] = 0.0;
   int rc = sbk::launch_add_node_blocks(sys->nn, sys->outer, sys->inner, sys->values, n, nodes_dev, blocks_dev,
-                                       sys->missing, st);
+                                       sys->host + 4, st);
   if (rc) return fail(SBK_ERR_CUDA, "add_node_blocks launch");
-  int32_t missing = 0;
-  SBK_CUDA(cudaMemcpyAsync(&missing, sys->missing, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   SBK_CUDA(cudaStreamSynchronize(st));
-  if (missing) return fail(SBK_ERR_ARGUMENT, "a node block names a node out of range or lies outside the pattern");
+  if (sys->host[4] != 0.0) return fail(SBK_ERR_ARGUMENT, "a node block names a node out of range or lies outside the pattern");
   return SBK_OK;
 }
 
@@ -985,7 +993,7 @@ int sbk_system_vjp_x(sbk_system* sys, const double* u_dev, const double* lambda_
                                     std::to_string(code) + ")");
   }
   rc = sbk::launch_assemble_forces(sys->maps(), sys->force, sys->energy_e, sys->yield, sys->p.nq, gx_dev, sys->scratch,
-                                   sys->scalars, st);
+                                   sys->scalars, nullptr, nullptr, st);
   if (rc) return fail(SBK_ERR_CUDA, "shape derivative gather");
   return SBK_OK;
 }

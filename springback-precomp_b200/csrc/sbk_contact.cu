@@ -205,7 +205,9 @@ __global__ void flag_count_kernel(int n, const uint8_t* __restrict__ flag, int32
 }
 
 // Exclusive offsets of nb block counts, in place; the total into *count.
-__global__ void block_offsets_kernel(int nb, int32_t* __restrict__ block_count, int32_t* __restrict__ count) {
+// total, if any: count[1] takes the total so far, which takes this count.
+__global__ void block_offsets_kernel(int nb, int32_t* __restrict__ block_count, int32_t* __restrict__ count,
+                                     int32_t* __restrict__ total) {
   __shared__ int32_t warp_sums[32];
   __shared__ int32_t carry;
   if (threadIdx.x == 0) carry = 0;
@@ -235,7 +237,13 @@ __global__ void block_offsets_kernel(int nb, int32_t* __restrict__ block_count, 
     if (threadIdx.x == 0) carry += warp_sums[(blockDim.x >> 5) - 1];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *count = carry;
+  if (threadIdx.x == 0) {
+    *count = carry;
+    if (total) {
+      count[1] = *total;
+      *total += carry;
+    }
+  }
 }
 
 __global__ void flag_place_kernel(int n, const uint8_t* __restrict__ flag, const int32_t* __restrict__ block_offset,
@@ -260,14 +268,14 @@ __global__ void flag_place_kernel(int n, const uint8_t* __restrict__ flag, const
 }
 
 void ordered_compact(int n, const uint8_t* flag, int32_t* out, int32_t* count, int32_t* block_scratch,
-                     cudaStream_t st) {
+                     cudaStream_t st, int32_t* total = nullptr) {
   const int nb = (n + kCompactBlock - 1) / kCompactBlock;
   if (nb == 0) {
     cudaMemsetAsync(count, 0, sizeof(int32_t), st);
     return;
   }
   flag_count_kernel<<<nb, kCompactBlock, 0, st>>>(n, flag, block_scratch);
-  block_offsets_kernel<<<1, 1024, 0, st>>>(nb, block_scratch, count);
+  block_offsets_kernel<<<1, 1024, 0, st>>>(nb, block_scratch, count, total);
   flag_place_kernel<<<nb, kCompactBlock, 0, st>>>(n, flag, block_scratch, out);
 }
 
@@ -435,9 +443,10 @@ __global__ void evaluate_kernel(DTool t, int nslaves, const int32_t* __restrict_
 __global__ void scatter_kernel(int nslots, const int32_t* __restrict__ list, const int32_t* __restrict__ nlist,
                                EvalOut ev, double* __restrict__ residual, double* __restrict__ gross,
                                double* __restrict__ positions, int32_t* __restrict__ block_nodes,
-                               double* __restrict__ blocks, int base, int want_tangent, int32_t* __restrict__ asym) {
+                               double* __restrict__ blocks, int want_tangent, int32_t* __restrict__ asym) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= *nlist) return;
+  const int base = nlist[1];  // the blocks of the tools before
   const int slot = list[k];
   const int64_t node = ev.node[slot];
   for (int c = 0; c < 3; ++c) {
@@ -500,6 +509,7 @@ __global__ void resultant_kernel(const int32_t* __restrict__ list, const int32_t
 // same sums in the same order every call): kNormBlocks blocks of partial
 // sums of squares, then one block over the partials.
 constexpr int kNormBlocks = 296;
+constexpr int kHostRes = 6;  // of the host's doubles: norms 3, flags 3, then the tool sums
 
 __global__ void norms_partial_kernel(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                                      const double* __restrict__ c, double* __restrict__ partial) {
@@ -521,7 +531,10 @@ __global__ void norms_partial_kernel(int64_t n, const double* __restrict__ a, co
     for (int k = 0; k < 3; ++k) partial[3 * blockIdx.x + k] = sh[0][k];
 }
 
-__global__ void norms_kernel(int nb, const double* __restrict__ partial, double* __restrict__ out) {
+// The norms, the flags and block count, and the n tool sums into the host's
+// page-locked memory (kHostRes, ...): one synchronisation reads them all.
+__global__ void norms_kernel(int nb, const double* __restrict__ partial, const int32_t* __restrict__ flags, int n,
+                             const double* __restrict__ res, double* __restrict__ host) {
   __shared__ double sh[256][3];
   double s[3] = {0, 0, 0};
   for (int i = threadIdx.x; i < nb; i += blockDim.x)
@@ -534,7 +547,11 @@ __global__ void norms_kernel(int nb, const double* __restrict__ partial, double*
     __syncthreads();
   }
   if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) out[k] = sqrt(sh[0][k]);
+    for (int k = 0; k < 3; ++k) {
+      host[k] = sqrt(sh[0][k]);
+      host[3 + k] = (double)flags[k];
+    }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) host[kHostRes + i] = res[i];
 }
 
 // ToolContact::anticipate for one tool (RigidTool.cpp:557-603).
@@ -614,7 +631,7 @@ struct HostTool {
   double* epen = nullptr;
   double* epscale = nullptr;
   int32_t* alist = nullptr;
-  int32_t* nalist = nullptr;
+  int32_t* nalist = nullptr;    // its length; the blocks of the tools before
   int32_t* cblocks = nullptr;   // ordered compaction: per-block counts
   // The uniform-grid hash of the slave nodes (rebuilt each increment).
   uint32_t gmask = 0;           // table size - 1 (a power of two)
@@ -673,8 +690,11 @@ struct sbk_contact {
   double* blocks = nullptr;
   int capacity = 0;  // blocks
   int num_blocks = 0;
-  int32_t* flags = nullptr;  // [0] failed, [1] asym
-  double* norms = nullptr;
+  // residual, gross and positions lie in one allocation with what else each
+  // evaluate starts from zero: res_dev, flags, the tools' largest motions.
+  size_t zeroed = 0;         // its doubles
+  int32_t* flags = nullptr;  // [0] failed, [1] asym, [2] blocks so far
+  double* host = nullptr;    // page-locked: norms, flags, tool sums
   double* norm_partial = nullptr;  // 3 per block of the norms' first stage
   double* res_dev = nullptr;  // 6 per tool
   std::vector<double> resultants;
@@ -693,15 +713,15 @@ int calloc_dev(T** p, size_t n) {
 void free_contact(sbk_contact* c) {
   for (HostTool& t : c->tools) {
     void* ptrs[] = {t.nodes, t.area, t.kappa, t.cflag, t.cand, t.ncand, t.h_flag, t.h_force, t.h_rel, t.t_flag,
-                    t.t_force, t.t_rel, t.moved, t.act, t.slip, t.enode, t.eforce, t.ek, t.epen, t.epscale,
+                    t.t_force, t.t_rel, t.act, t.slip, t.enode, t.eforce, t.ek, t.epen, t.epscale,
                     t.alist, t.nalist, t.cblocks, t.gkey, t.gcount, t.gstart, t.gbinned, t.gscan};
     for (void* p : ptrs)
       if (p) cudaFree(p);
   }
-  void* ptrs[] = {c->coords, c->start, c->residual, c->gross, c->positions, c->block_nodes, c->blocks, c->flags,
-                  c->norms, c->norm_partial, c->res_dev};
+  void* ptrs[] = {c->coords, c->start, c->residual, c->block_nodes, c->blocks, c->norm_partial};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (c->host) cudaFreeHost(c->host);
   delete c;
 }
 double norm3h(const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); }
@@ -737,11 +757,22 @@ int sbk_contact_create(const sbk_mesh* mesh, int32_t num_tools, const sbk_tool* 
     return cfail(SBK_ERR_CUDA, "coordinate upload");
   }
   TRYC(calloc_dev(&c->start, 3 * c->nn));
-  TRYC(calloc_dev(&c->residual, 3 * c->nn));
-  TRYC(calloc_dev(&c->gross, 3 * c->nn));
-  TRYC(calloc_dev(&c->positions, 3 * c->nn));
-  TRYC(calloc_dev(&c->flags, 4));
-  TRYC(calloc_dev(&c->norms, 4));
+  {
+    const size_t nd = 3 * static_cast<size_t>(c->nn), nt = std::max(1, num_tools);
+    c->zeroed = 3 * nd + 6 * nt + 2 + nt;
+    TRYC(calloc_dev(&c->residual, c->zeroed));
+    c->gross = c->residual + nd;
+    c->positions = c->gross + nd;
+    c->res_dev = c->positions + nd;
+    c->flags = reinterpret_cast<int32_t*>(c->res_dev + 6 * nt);
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&c->host), (kHostRes + 6 * nt) * sizeof(double),
+                                        cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      c->host = nullptr;
+      free_contact(c);
+      return cfail(SBK_ERR_CUDA, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+    }
+  }
   TRYC(calloc_dev(&c->norm_partial, 3 * kNormBlocks));
   int total = 0;
   for (int k = 0; k < num_tools; ++k) {
@@ -811,7 +842,7 @@ int sbk_contact_create(const sbk_mesh* mesh, int32_t num_tools, const sbk_tool* 
     TRYC(calloc_dev(&h.t_flag, n));
     TRYC(calloc_dev(&h.t_force, 3 * n));
     TRYC(calloc_dev(&h.t_rel, 3 * n));
-    TRYC(calloc_dev(&h.moved, 1));
+    h.moved = reinterpret_cast<unsigned long long*>(c->flags + 4) + k;
     TRYC(calloc_dev(&h.act, n));
     TRYC(calloc_dev(&h.slip, n));
     TRYC(calloc_dev(&h.enode, n));
@@ -820,7 +851,7 @@ int sbk_contact_create(const sbk_mesh* mesh, int32_t num_tools, const sbk_tool* 
     TRYC(calloc_dev(&h.epen, n));
     TRYC(calloc_dev(&h.epscale, n));
     TRYC(calloc_dev(&h.alist, n));
-    TRYC(calloc_dev(&h.nalist, 1));
+    TRYC(calloc_dev(&h.nalist, 2));
     TRYC(calloc_dev(&h.cblocks, (n + kCompactBlock - 1) / kCompactBlock + 1));
     {
       size_t table = 1024;
@@ -848,7 +879,6 @@ int sbk_contact_create(const sbk_mesh* mesh, int32_t num_tools, const sbk_tool* 
   c->capacity = std::max(1, total);
   TRYC(calloc_dev(&c->block_nodes, c->capacity));
   TRYC(calloc_dev(&c->blocks, 9 * static_cast<size_t>(c->capacity)));
-  TRYC(calloc_dev(&c->res_dev, 6 * std::max<size_t>(1, c->tools.size())));
 #undef TRYC
   c->t0 = c->tools.empty() ? 0.0 : c->tools.front().times.front();
   c->margin = __builtin_inf();
@@ -962,13 +992,7 @@ int sbk_contact_evaluate(sbk_contact* c, const double* u_dev, double t, int want
   cudaStream_t st = c->stream;
   std::memset(out, 0, sizeof(*out));
   const size_t nd = 3 * static_cast<size_t>(c->nn);
-  SBK_C(cudaMemsetAsync(c->residual, 0, nd * sizeof(double), st));
-  SBK_C(cudaMemsetAsync(c->gross, 0, nd * sizeof(double), st));
-  SBK_C(cudaMemsetAsync(c->positions, 0, nd * sizeof(double), st));
-  SBK_C(cudaMemsetAsync(c->flags, 0, 4 * sizeof(int32_t), st));
-  SBK_C(cudaMemsetAsync(c->res_dev, 0, 6 * std::max<size_t>(1, c->tools.size()) * sizeof(double), st));
-  std::vector<int32_t> counts(c->tools.size(), 0);
-  int base = 0;
+  SBK_C(cudaMemsetAsync(c->residual, 0, c->zeroed * sizeof(double), st));
   for (size_t k = 0; k < c->tools.size(); ++k) {
     HostTool& h = c->tools[k];
     double cc[3];
@@ -978,34 +1002,28 @@ int sbk_contact_evaluate(sbk_contact* c, const double* u_dev, double t, int want
     if (!c->active[k] || h.nslaves == 0) continue;
     double c0[3];
     h.position(c->t0, c0);
-    SBK_C(cudaMemsetAsync(h.moved, 0, sizeof(unsigned long long), st));
     const int blocks = (h.nslaves + 127) / 128;
     moved_kernel<<<blocks, 128, 0, st>>>(h.nslaves, h.nodes, u_dev, c->start, h.moved);
     evaluate_kernel<<<blocks, 128, 0, st>>>(h.d, h.nslaves, h.nodes, h.area, h.kappa, h.cand, h.ncand, h.moved,
                                             c->margin, c->coords, u_dev, c->start, cc[0], cc[1], cc[2], c0[0],
                                             c0[1], c0[2], c->friction_tangent, h.h_flag, h.h_force, h.h_rel,
                                             h.t_flag, h.t_force, h.t_rel, h.ev(), c->flags);
-    ordered_compact(h.nslaves, h.act, h.alist, h.nalist, h.cblocks, st);
-    // The block offset of this tool needs the count of the previous ones.
-    SBK_C(cudaMemcpyAsync(&counts[k], h.nalist, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    SBK_C(cudaStreamSynchronize(st));
+    ordered_compact(h.nslaves, h.act, h.alist, h.nalist, h.cblocks, st, c->flags + 2);
     scatter_kernel<<<(h.nslaves + 127) / 128, 128, 0, st>>>(h.nslaves, h.alist, h.nalist, h.ev(), c->residual,
-                                                            c->gross, c->positions, c->block_nodes, c->blocks, base,
+                                                            c->gross, c->positions, c->block_nodes, c->blocks,
                                                             want_tangent, c->flags + 1);
     resultant_kernel<<<1, 256, 0, st>>>(h.alist, h.nalist, h.ev(), c->res_dev + 6 * k);
-    if (want_tangent) base += counts[k];
   }
   norms_partial_kernel<<<kNormBlocks, 256, 0, st>>>(static_cast<int64_t>(nd), c->gross, c->positions, c->residual,
                                                    c->norm_partial);
-  norms_kernel<<<1, 256, 0, st>>>(kNormBlocks, c->norm_partial, c->norms);
+  norms_kernel<<<1, 256, 0, st>>>(kNormBlocks, c->norm_partial, c->flags, static_cast<int>(6 * c->tools.size()),
+                                  c->res_dev, c->host);
   SBK_C(cudaGetLastError());
-  double norms[3];
-  int32_t flags[2];
-  std::vector<double> res(6 * std::max<size_t>(1, c->tools.size()));
-  SBK_C(cudaMemcpyAsync(norms, c->norms, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  SBK_C(cudaMemcpyAsync(flags, c->flags, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  SBK_C(cudaMemcpyAsync(res.data(), c->res_dev, res.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   SBK_C(cudaStreamSynchronize(st));
+  const double* norms = c->host;
+  const double* res = c->host + kHostRes;
+  const bool failed = c->host[3] != 0.0;
+  const int base = want_tangent ? static_cast<int>(c->host[5]) : 0;
   for (size_t k = 0; k < c->tools.size(); ++k) {
     for (int i = 0; i < 3; ++i) c->resultants[9 * k + 3 + i] = res[6 * k + i];
     c->resultants[9 * k + 6] = res[6 * k + 3];
@@ -1017,12 +1035,12 @@ int sbk_contact_evaluate(sbk_contact* c, const double* u_dev, double t, int want
   out->block_nodes_dev = c->block_nodes;
   out->blocks_dev = c->blocks;
   out->num_blocks = base;
-  out->symmetric = flags[1] ? 0 : 1;
+  out->symmetric = c->host[4] != 0.0 ? 0 : 1;
   out->gross = norms[0];
   out->round_off = norms[1];
   out->force_norm = norms[2];
-  out->failed = flags[0];
-  if (flags[0]) return cfail(SBK_ERR_SOLVER, "a node lies within half the radius of a tool: the tool is through the surface");
+  out->failed = failed ? 1 : 0;
+  if (failed) return cfail(SBK_ERR_SOLVER, "a node lies within half the radius of a tool: the tool is through the surface");
   return SBK_OK;
 }
 
@@ -1044,13 +1062,10 @@ int sbk_contact_anticipate(sbk_contact* c, const double* u_dev, const double* du
     double cc[3];
     h.position(t, cc);
     const int blocks = (h.nslaves + 127) / 128;
+    // Slots past the candidate count are never written: their flags clear.
+    SBK_C(cudaMemsetAsync(h.act, 0, h.nslaves, st));
     anticipate_kernel<<<blocks, 128, 0, st>>>(h.d, h.nodes, h.area, h.kappa, h.cand, h.ncand, c->coords, u_dev,
                                               du_dev, cc[0], cc[1], cc[2], h.act, h.ek, h.enode, h.eforce);
-    // Slots past the candidate count are never written: clear their flags.
-    int32_t nc = 0;
-    SBK_C(cudaMemcpyAsync(&nc, h.ncand, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    SBK_C(cudaStreamSynchronize(st));
-    if (nc < h.nslaves) SBK_C(cudaMemsetAsync(h.act + nc, 0, h.nslaves - nc, st));
     ordered_compact(h.nslaves, h.act, h.alist, h.nalist, h.cblocks, st);
     int32_t n = 0;
     SBK_C(cudaMemcpyAsync(&n, h.nalist, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

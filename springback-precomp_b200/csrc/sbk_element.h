@@ -71,10 +71,11 @@ struct GatherMaps {
 int launch_assemble_values(const GatherMaps& m, const double* tangent, double* values, cudaStream_t stream);
 // K2: f_int and the per-DOF gross sums from the element forces; the partial
 // sums of energy, gross^2 and the yield count into `scalars`
-// (double[3]: energy, gross^2, yielding).
+// (double[3]: energy, gross^2, yielding), and, where host is not null, into
+// host (4 doubles the device can write) with *first_failure.
 int launch_assemble_forces(const GatherMaps& m, const double* force, const double* energy_e,
                            const uint8_t* yield, int nq, double* internal, double* scratch, double* scalars,
-                           cudaStream_t stream);
+                           const int32_t* first_failure, double* host, cudaStream_t stream);
 size_t assemble_scratch_doubles();
 // Energy, gross, yielding points, lowest failing element (-1) and its code
 // into summary (5 doubles, device), from the reductions' scalars.
@@ -93,6 +94,6 @@ int launch_schedule(int64_t ne, int nq, const int32_t* iterations, const uint8_t
 size_t schedule_scratch_ints(int64_t ne);
 // add_node_block for n blocks, in list order.
 int launch_add_node_blocks(int64_t nn, const int32_t* outer, const int32_t* inner, double* values, int32_t n,
-                          const int32_t* nodes, const double* blocks, int32_t* missing, cudaStream_t stream);
+                          const int32_t* nodes, const double* blocks, double* missing, cudaStream_t stream);
 
 }  // namespace sbk

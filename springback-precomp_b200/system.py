@@ -38,7 +38,7 @@ class _DeviceView:
 
 def device_view(ptr: int, shape, dtype=torch.float64) -> torch.Tensor:
     typestr = {torch.float64: "<f8", torch.int32: "<i4", torch.uint8: "|u1"}[dtype]
-    if int(np.prod(shape)) == 0 or not ptr:
+    if not ptr or 0 in shape:
         return torch.empty(shape, dtype=dtype, device="cuda")
     return torch.as_tensor(_DeviceView(ptr, shape, typestr), device="cuda")
 
