@@ -13,14 +13,16 @@
 //   panel_kernel       factorises the next kPanel columns' diagonal block and
 //                      solves the rows below (every block factorises the
 //                      small block for itself rather than wait for one);
-//   tile_kernel        takes the panel's product off the rest, in 64 x 64
-//                      tiles on the FP64 tensor instruction;
+//   tile_kernel        takes the panel's product off the front's own columns
+//                      in 64 x 64 tiles on the FP64 tensor instruction and,
+//                      after the last panel, all its columns' product off
+//                      the remainder, which is so read and written once;
 //
 // and the solves walk the same levels with a block a front. What bounds it is
 // the chain of levels and panels, some hundred launches of a few microseconds
 // for a sheet of 13,689 rows. Measured there (41 x 41 x 3 nodes, clamped):
 // factorisation and solve 44.7 ms with the level-scheduled sparse Cholesky of
-// the library, 1.8 ms so (2.9 with a barrier in each of a panel's 32 steps).
+// the library, 1.6 ms so.
 #include "sbk_multifrontal.h"
 
 #include <algorithm>
@@ -72,7 +74,21 @@ __global__ void __launch_bounds__(32 * kAddColumns)
     }
     if (lo == rest || at[lo] != column) continue;
     const double* from = f.arena + f.offset[c] + (int64_t)(it.y + lo) * it.z + it.y;
-    for (int r = lo + lane; r < rest; r += 32) to[at[r]] += from[r];
+    // Four rows at once: the places differ, which the compiler cannot know.
+    for (int r0 = lo + lane; r0 < rest; r0 += 128) {
+      double* at4[4];
+      double sum[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = min(r0 + 32 * u, rest - 1);
+        at4[u] = to + at[r];
+        sum[u] = *at4[u] + from[r];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r0 + 32 * u < rest) *at4[u] = sum[u];
+    }
+    __syncwarp();
   }
 }
 
@@ -88,34 +104,38 @@ __global__ void __launch_bounds__(kRowChunk)
   const int4 me = f.front[task.x];
   const int m = me.z, nb = min(kPanel, me.y - p0), tid = threadIdx.x;
   double* A = f.arena + f.offset[task.x];
+  const int row = task.y + tid;
+  double x[kPanel];
+#pragma unroll
+  for (int j = 0; j < kPanel; ++j) x[j] = j < nb && row < m ? A[(int64_t)(p0 + j) * m + row] : 0.0;
   {
     // Every warp the whole block for itself, lane r the row r (identity
     // beyond nb): no barrier in the 32 steps.
     const int r = tid & 31;
-    double row[kPanel];
+    double d_row[kPanel];
 #pragma unroll
     for (int c = 0; c < kPanel; ++c)
-      row[c] = r < nb && c <= r ? A[(int64_t)(p0 + c) * m + p0 + r] : (r == c ? 1.0 : 0.0);
+      d_row[c] = r < nb && c <= r ? A[(int64_t)(p0 + c) * m + p0 + r] : (r == c ? 1.0 : 0.0);
     int bad = 0x7fffffff;
     double mine = 1.0;
 #pragma unroll
     for (int j = 0; j < kPanel; ++j) {
-      double d = __shfl_sync(0xffffffffu, row[j], j);
+      double d = __shfl_sync(0xffffffffu, d_row[j], j);
       if (!(d > 0.0)) {
         bad = min(bad, j);
         d = 1.0;
       }
       const double scale = rsqrt(d);
-      const double l = row[j] * scale;
+      const double l = d_row[j] * scale;
       if (r == j) mine = scale;
-      row[j] = r == j ? d * scale : l;
+      d_row[j] = r == j ? d * scale : l;
 #pragma unroll
-      for (int c = j + 1; c < kPanel; ++c) row[c] -= l * __shfl_sync(0xffffffffu, l, c);
+      for (int c = j + 1; c < kPanel; ++c) d_row[c] -= l * __shfl_sync(0xffffffffu, l, c);
     }
     if (bad < nb && tid == 0) atomicMin(failed, me.x + p0 + bad);
     if (tid < 32) {
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c) L[r][c] = c <= r ? row[c] : 0.0;
+      for (int c = 0; c < kPanel; ++c) L[r][c] = c <= r ? d_row[c] : 0.0;
       inv[r] = mine;
     }
     __syncthreads();
@@ -124,11 +144,7 @@ __global__ void __launch_bounds__(kRowChunk)
     double* D = diag + (int64_t)(diag_offset[task.x] + p0 / kPanel) * kPanel * kPanel;
     for (int i = tid; i < kPanel * kPanel; i += kRowChunk) D[i] = L[i % kPanel][i / kPanel];
   }
-  const int row = task.y + tid;
   if (row >= m) return;
-  double x[kPanel];
-#pragma unroll
-  for (int j = 0; j < kPanel; ++j) x[j] = j < nb ? A[(int64_t)(p0 + j) * m + row] : 0.0;
 #pragma unroll
   for (int j = 0; j < kPanel; ++j) {
     if (j < nb) {
@@ -148,44 +164,24 @@ __device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// C -= P_i P_j^T of one 64 x 64 tile of the lower trailing matrix: four warps
-// a quadrant of 4 x 4 tensor tiles each.
+// C -= P_i P_j^T of one 64 x 64 tile of the lower matrix below the columns P:
+// four warps a quadrant of 4 x 4 tensor tiles each. P is the panel at p0 and C
+// the front's own columns, or (p0 < 0) P all its columns and C the remainder.
 __global__ void __launch_bounds__(128)
     tile_kernel(Fronts f, const int4* __restrict__ tasks, int p0) {
   __shared__ double P[2][kPanel][kTile + 4];
   const int4 task = tasks[blockIdx.x];
   const int4 me = f.front[task.x];
-  const int m = me.z, nb = min(kPanel, me.y - p0), base = p0 + nb;
+  const int m = me.z, first = p0 < 0 ? 0 : p0, base = p0 < 0 ? me.y : min(p0 + kPanel, me.y);
+  const int columns = p0 < 0 ? m : me.y;
   double* A = f.arena + f.offset[task.x];
   const int r0 = base + task.y * kTile, c0 = base + task.z * kTile;
-  for (int i = threadIdx.x; i < kPanel * kTile; i += 128) {
-    const int r = i % kTile, j = i / kTile;
-    const double* col = A + (int64_t)(p0 + j) * m;
-    P[0][j][r] = j < nb && r0 + r < m ? col[r0 + r] : 0.0;
-    P[1][j][r] = j < nb && c0 + r < m ? col[c0 + r] : 0.0;
-  }
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
-  if (r0 + wr + 31 < c0 + wc) return;  // above the diagonal
+  const bool lower = r0 + wr + 31 >= c0 + wc;
+  // C first, all of it in flight at once: added at the end instead, each entry
+  // waits for the store before it (17 us a tile for 6).
   double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-#pragma unroll
-  for (int k = 0; k < kPanel; k += 4) {
-    double a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a[i] = P[0][k + t][wr + 8 * i + g];
-      b[i] = P[1][k + t][wc + 8 * i + g];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) mma884(acc[i][j], a[i], b[j]);
-  }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -193,7 +189,43 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const int row = r0 + wr + 8 * i + g, col = c0 + wc + 8 * j + 2 * t + s;
-        if (row < m && col <= row) A[(int64_t)col * m + row] -= acc[i][j][s];
+        acc[i][j][s] = row < m && col < columns && col <= row ? A[(int64_t)col * m + row] : 0.0;
+      }
+#pragma unroll 1
+  for (int k0 = first; k0 < base; k0 += kPanel) {
+    if (k0 > first) __syncthreads();
+#pragma unroll
+    for (int i = threadIdx.x; i < kPanel * kTile; i += 128) {
+      const int r = i % kTile, j = i / kTile;
+      const double* col = A + (int64_t)(k0 + j) * m;
+      P[0][j][r] = k0 + j < base && r0 + r < m ? col[r0 + r] : 0.0;
+      P[1][j][r] = k0 + j < base && c0 + r < m ? col[c0 + r] : 0.0;
+    }
+    __syncthreads();
+    if (!lower) continue;
+#pragma unroll
+    for (int k = 0; k < kPanel; k += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i] = -P[0][k + t][wr + 8 * i + g];
+        b[i] = P[1][k + t][wc + 8 * i + g];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma884(acc[i][j], a[i], b[j]);
+    }
+  }
+  if (!lower) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int row = r0 + wr + 8 * i + g, col = c0 + wc + 8 * j + 2 * t + s;
+        if (row < m && col < columns && col <= row) A[(int64_t)col * m + row] = acc[i][j][s];
       }
 }
 
@@ -597,13 +629,21 @@ cudaError_t Multifrontal::build(const FrontOrder& order, const std::vector<int32
           panel_tasks.push_back(make_int2(f, r));
           r += kRowChunk;
         } while (r < t.z);
-        const int tiles = (t.z - base + kTile - 1) / kTile;
+        const int tiles = (t.z - base + kTile - 1) / kTile, own = (t.y - base + kTile - 1) / kTile;
         for (int i = 0; i < tiles; ++i)
-          for (int j = 0; j <= i; ++j) tile_tasks.push_back(make_int4(f, i, j, 0));
+          for (int j = 0; j <= i && j < own; ++j) tile_tasks.push_back(make_int4(f, i, j, 0));
       }
       L.panels.push_back((int)panel_tasks.size() - L.panel0.back());
       L.tiles.push_back((int)tile_tasks.size() - L.tile0.back());
     }
+    L.rest0 = (int)tile_tasks.size();
+    for (int f : members[(size_t)l]) {
+      const int4& t = front[(size_t)f];
+      const int tiles = (t.z - t.y + kTile - 1) / kTile;
+      for (int i = 0; i < tiles; ++i)
+        for (int j = 0; j <= i; ++j) tile_tasks.push_back(make_int4(f, i, j, 0));
+    }
+    L.rest = (int)tile_tasks.size() - L.rest0;
   }
   cudaError_t err = upload(&front_, front);
   auto next = [&](cudaError_t e) {
@@ -657,6 +697,7 @@ cudaError_t Multifrontal::factor(const double* values, int32_t* failed, cudaStre
                                                           failed);
       if (L.tiles[s]) tile_kernel<<<L.tiles[s], 128, 0, stream>>>(f, tile_tasks_ + L.tile0[s], p0);
     }
+    if (L.rest) tile_kernel<<<L.rest, 128, 0, stream>>>(f, tile_tasks_ + L.rest0, -1);
   }
   return cudaGetLastError();
 }

@@ -51,6 +51,7 @@ class Multifrontal {
     int front0 = 0, fronts = 0;         // of the fronts in level order
     int adds = 0, adds0 = 0;            // extend-add tasks
     std::vector<int> panel0, panels, tile0, tiles;  // per panel step
+    int rest = 0, rest0 = 0;            // tiles of the remainders
   };
   template <class T>
   cudaError_t upload(T** out, const std::vector<T>& in);
