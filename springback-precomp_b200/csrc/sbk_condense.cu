@@ -7,10 +7,12 @@
 // a chain of small contractions, and goes in 8 x 8 tiles through the FP64
 // tensor instruction: at a quarter of the instructions of the same products
 // in FMAs it is the one form that keeps the FP64 pipe, not the issue slots,
-// the limit. Column 33 carries the stress, so that f_u comes with K_ua.
-// Measured on 1,000,000 elements (2 x 2 x 2 points, non-symmetric): 17.8 ms as
-// FMAs of 8 lanes an element, 12.2 ms so; the tensor instructions alone are
-// 7 ms of it.
+// the limit. The 33rd degree of freedom and the stress (f_u) would each open
+// a tile of one column or row: they go as FMAs, four lanes an entry. Measured
+// on 1,000,000 elements (2 x 2 x 2 points, non-symmetric): 17.8 ms as FMAs of
+// 8 lanes an element, 12.4 ms all in tiles, 11.4 ms so; the tensor
+// instructions alone are 5.5 ms of it. Four blocks an SM (spilling at 128
+// registers) take 12.0 ms, two points unrolled 12.1.
 #include <cuda_runtime.h>
 
 #include "sbk_element_math.cuh"
@@ -63,13 +65,14 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
   const double* own = rec + own_at(nq);
   const int g = lane >> 2, t = lane & 3;
   const bool small = p.kinematics == SBK_SMALL_STRAIN;
-  double uu[3][3][2], ua[3][2][2], au[2][3][2], geo[2][2];
+  // Column 32 of K_ua, f_u and row 32 of K_au beyond the tiles: a lane's
+  // share over its components, four lanes an entry.
+  double uu[3][3][2], ua[3][2], au[3][2], last[3], fu[3], lastrow[3], geo[2][2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
 #pragma unroll
     for (int j = 0; j < 3; ++j) uu[i][j][0] = uu[i][j][1] = 0.0;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) ua[i][j][0] = ua[i][j][1] = au[j][i][0] = au[j][i][1] = 0.0;
+    ua[i][0] = ua[i][1] = au[i][0] = au[i][1] = last[i] = fu[i] = lastrow[i] = 0.0;
   }
   geo[0][0] = geo[0][1] = geo[1][0] = geo[1][1] = 0.0;
   // The lane's strain components: c(t, 0) the normal one t, c(t, 1) the
@@ -88,8 +91,8 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
   int fo[5], go[5];
 #pragma unroll
   for (int i = 0; i < 5; ++i) {
-    const int dof = 8 * i + g;
-    const bool live = dof < 33 && t < 3;
+    const int dof = i < 4 ? 8 * i + g : 32;  // the last in every row
+    const bool live = t < 3;
     fo[i] = live ? kTabF + 5 * (dof % 3) + t : kTabZero;
     go[i] = live ? 5 * (dof / 3) + t : 0;
   }
@@ -144,17 +147,14 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
         mma884(db[i], bf[i][0], d0);
         mma884(db[i], bf[i][1], d1);
       }
-      if (g == 1) {  // column 33: the stress
-        db[4][0] = t < 3 ? w * R[s0] : 0.0;
-        db[4][1] = t < 3 ? w * R[s1] : 0.0;
+      const double sn = t < 3 ? w * R[s0] : 0.0, ss = t < 3 ? w * R[s1] : 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        mma884(ua[i], bf[i][0], db[3][0]);
+        mma884(ua[i], bf[i][1], db[3][1]);
+        last[i] = fma(bf[i][1], db[4][1], fma(bf[i][0], db[4][0], last[i]));
+        fu[i] = fma(bf[i][1], ss, fma(bf[i][0], sn, fu[i]));
       }
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          mma884(ua[i][j], bf[i][0], db[3 + j][0]);
-          mma884(ua[i][j], bf[i][1], db[3 + j][1]);
-        }
       if (TANGENT) {
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -165,12 +165,11 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
           }
         if (!SYM) {
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              mma884(au[i][j], bf[3 + i][0], db[j][0]);
-              mma884(au[i][j], bf[3 + i][1], db[j][1]);
-            }
+          for (int j = 0; j < 3; ++j) {
+            mma884(au[j], bf[3][0], db[j][0]);
+            mma884(au[j], bf[3][1], db[j][1]);
+            lastrow[j] = fma(bf[4][1], db[j][1], fma(bf[4][0], db[j][0], lastrow[j]));
+          }
         }
       }
       if (!small) {
@@ -198,16 +197,27 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
   for (int i = 0; i < 3; ++i) {
     const int row = 8 * i + g, a3 = row / 3, k3 = row - 3 * a3;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int o = 1; o <= 2; o <<= 1) {
+      last[i] += __shfl_xor_sync(0xffffffffu, last[i], o);
+      fu[i] += __shfl_xor_sync(0xffffffffu, fu[i], o);
+      if (!SYM && TANGENT) lastrow[i] += __shfl_xor_sync(0xffffffffu, lastrow[i], o);
+    }
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const int col = 8 * j + 2 * t + s;
-        if (col < 10) {
-          const double v = ua[i][j][s] + (col < 9 && col % 3 == k3 ? gs[a3 * 11 + 8 + col / 3] : 0.0);
-          x[kKua + row * 10 + col] = v;
-          if (SYM && TANGENT && col < 9) x[kC + col * 25 + row] = v;
-        }
-      }
+    for (int s = 0; s < 2; ++s) {
+      const int col = 2 * t + s;
+      const double v = ua[i][s] + (col % 3 == k3 ? gs[a3 * 11 + 8 + col / 3] : 0.0);
+      x[kKua + row * 10 + col] = v;
+      if (SYM && TANGENT) x[kC + col * 25 + row] = v;
+    }
+    const double mode = k3 == 2 ? gs[a3 * 11 + 10] : 0.0;  // entry 32's
+    if (t == 0) {
+      x[kKua + row * 10 + 8] = last[i] + mode;
+      if (SYM && TANGENT) x[kC + 8 * 25 + row] = last[i] + mode;
+    } else if (t == 1) {
+      x[kKua + row * 10 + 9] = fu[i];
+    } else if (t == 2 && !SYM && TANGENT) {
+      x[kC + 8 * 25 + row] = lastrow[i] + mode;
+    }
   }
   if (!SYM && TANGENT) {
 #pragma unroll
@@ -215,11 +225,7 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const int col = 8 * j + 2 * t + s, a3 = col / 3, k3 = col - 3 * a3;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int row = 8 * i + g;
-          if (row < 9) x[kC + row * 25 + col] = au[i][j][s] + (row % 3 == k3 ? gs[a3 * 11 + 8 + row / 3] : 0.0);
-        }
+        x[kC + g * 25 + col] = au[j][s] + (g % 3 == k3 ? gs[a3 * 11 + 8 + g / 3] : 0.0);
       }
   }
   if (lane < 9) x[kC + lane * 25 + 24] = own[kCondR + lane];
