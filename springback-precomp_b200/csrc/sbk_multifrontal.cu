@@ -22,7 +22,7 @@
 // the chain of levels and panels, some hundred launches of a few microseconds
 // for a sheet of 13,689 rows. Measured there (41 x 41 x 3 nodes, clamped):
 // factorisation and solve 44.7 ms with the level-scheduled sparse Cholesky of
-// the library, 1.6 ms so.
+// the library, 1.5 ms so.
 #include "sbk_multifrontal.h"
 
 #include <algorithm>
@@ -256,14 +256,25 @@ __global__ void __launch_bounds__(kSolveThreads)
     for (int i = tid; i < that.z - that.y; i += kSolveThreads) y[at[i]] += yc[i];
     __syncthreads();
   }
-  for (int p0 = 0; p0 < k; p0 += kPanel) {
-    const int nb = min(kPanel, k - p0);
-    if (tid < 32) {
-      const double* D = diag + (int64_t)(diag_offset[s] + p0 / kPanel) * kPanel * kPanel;
-      double l[kPanel], v = tid < nb ? y[p0 + tid] : 0.0;
-      const double inv = 1.0 / D[tid * kPanel + tid];
+  // Everything a panel reads but y is on its way before the barrier it waits
+  // for: the next triangle, the thread's first row.
+  double l[kPanel], inv = 0.0;
+  auto triangle = [&](int p0) {
+    if (tid >= 32) return;
+    const double* D = diag + (int64_t)(diag_offset[s] + p0 / kPanel) * kPanel * kPanel;
 #pragma unroll
-      for (int j = 0; j < kPanel; ++j) l[j] = D[j * kPanel + tid];  // L(tid, j)
+    for (int j = 0; j < kPanel; ++j) l[j] = D[j * kPanel + tid];  // L(tid, j)
+    inv = 1.0 / D[tid * kPanel + tid];
+  };
+  triangle(0);
+  for (int p0 = 0; p0 < k; p0 += kPanel) {
+    const int nb = min(kPanel, k - p0), first = p0 + nb + tid;
+    const double* row = A + (int64_t)p0 * m + first;
+    double a[kPanel];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) a[j] = j < nb && first < m ? row[(int64_t)j * m] : 0.0;
+    if (tid < 32) {
+      double v = tid < nb ? y[p0 + tid] : 0.0;
 #pragma unroll
       for (int j = 0; j < kPanel; ++j) {
         const double xj = __shfl_sync(0xffffffffu, v * inv, j);
@@ -272,16 +283,17 @@ __global__ void __launch_bounds__(kSolveThreads)
       x[tid] = v;
       if (tid < nb) y[p0 + tid] = v;
     }
+    if (p0 + kPanel < k) triangle(p0 + kPanel);
     __syncthreads();
-    for (int i = p0 + nb + tid; i < m; i += kSolveThreads) {
-      double v[4] = {0.0, 0.0, 0.0, 0.0};
-      const double* row = A + (int64_t)p0 * m + i;
-      if (nb == kPanel) {
+    for (int i = first; i < m; i += kSolveThreads) {
+      if (i > first) {
+        row += kSolveThreads;
 #pragma unroll
-        for (int j = 0; j < kPanel; ++j) v[j & 3] += row[(int64_t)j * m] * x[j];
-      } else {
-        for (int j = 0; j < nb; ++j) v[0] += row[(int64_t)j * m] * x[j];
+        for (int j = 0; j < kPanel; ++j) a[j] = j < nb ? row[(int64_t)j * m] : 0.0;
       }
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int j = 0; j < kPanel; ++j) v[j & 3] += a[j] * x[j];
       y[i] -= (v[0] + v[1]) + (v[2] + v[3]);
     }
     __syncthreads();
