@@ -55,6 +55,14 @@ METRIC = "Hex8 tangent+residual+assembly elem/s (FP64)"
 # 1.71 GB (the tile kernel 0.63, the condensation 0.69, the single kernel's
 # share 0.38); the traffic grows with the elements.
 K1_DRAM_BYTES_PER_ELEMENT = 1.706e9 / 80000
+
+
+def record_chunks(ne):
+    """Launches of K1's tile kernel: one per GiB of records (704 doubles an
+    element of 8 points)."""
+    return -(-ne // ((1 << 30) // (704 * 8)))
+
+
 # The single kernel (--local-iteration single): 0.69 + 5.28 GB in one launch
 # at 80,000 elements.
 K1_SINGLE_DRAM_BYTES_PER_ELEMENT = (0.692594688e9 + 5.275133e9) / 80000
@@ -778,11 +786,11 @@ def run_cone(args, rank, world):
             "contact": {"begin_grid_ms": grid_ms, "begin_scan_ms": scan_ms, "candidates": grid_cand,
                         "active": [int(cev.tools[k][6]) for k in range(2)],
                         "slaves": [int(len(t["nodes"])) for t in prob.tools], "margin_m": margin},
-            # K1 (the tile kernel, the condensation, the single kernel's list),
-            # K2b + finish, K2a; per tool 7 contact kernels (moved points,
+            # K1 (the tile kernel and the condensation per GiB of records, the
+            # single kernel's list), K2b + finish, K2a; per tool 7 contact kernels (moved points,
             # evaluate, the ordered compaction's 3, scatter, resultants), the
             # norms' two stages over both tools, and the blocks' add.
-            "gpu_launches": args.steps * (3 + 3 + 2 * 7 + 2 + 1), "clocks": clocks.summary(),
+            "gpu_launches": args.steps * (2 * record_chunks(ne) + 1 + 3 + 2 * 7 + 2 + 1), "clocks": clocks.summary(),
             "yielding_fraction": ev.yielding_points / (8.0 * ne),
             "setup_s": setup_s}
     print(json.dumps(line), flush=True)
@@ -1149,15 +1157,17 @@ def main():
                                       prob.mesh.gather(prob.u), committed, prob.alpha)
             flops_per_element = cnt / prob.mesh.num_elements
         el_ms = statistics.mean(elem_ms)
-        # Kernels of one step: K1 (the tile kernel and the condensation per GiB
-        # of records, 614 doubles an element, and the single kernel for the
-        # elements handed on; or one launch), then the force gather and its
-        # finish (2), the value gather, and for the single kernel the schedule
-        # (count, CUB's scan, place).
+        # Kernels of one step: K1 (two kernels per GiB of records, 704
+        # doubles an element; for the incompatible-mode Hex8 also the single
+        # kernel for the elements handed on, or in its place one launch and
+        # the schedule's count, scan and place), then the force gather and its
+        # finish (2) and the value gather.
         phases = args.element == "incompatible_modes" and args.local_iteration == "phases"
-        launches_per_step = (2 * -(-ne // ((1 << 30) // (614 * 8))) + 1 if phases else 1 + 3) + 3
+        standard = args.element != "incompatible_modes"
+        chunks = record_chunks(ne)
+        launches_per_step = (2 * chunks if standard else 2 * chunks + 1 if phases else 1 + 3) + 3
         k1_name = ("K1: the local iteration in tiles (tile_kernel, condense_kernel, element_list_kernel)" if phases else
-                   "element_kernel (K1)" if args.element == "incompatible_modes" else "standard_kernel (K1s)")
+                   "K1s: standard_points_kernel, standard_tangent_kernel" if standard else "element_kernel (K1)")
         roofline = None
         if flops_per_element:
             achieved = flops_per_element * ne / (el_ms / 1e3) / 1e12

@@ -184,8 +184,8 @@ int sbk_system_set_elements_per_block(sbk_system* sys, int elements_per_block);
  * elements whose K_aa turns indefinite or whose line search fails are handed
  * to the single kernel. Every rule.
  * SBK_LOCAL_SINGLE_KERNEL: one kernel runs each element from start to
- * finish. The first keeps records of up to 1 GiB on the device (4.9 KB an
- * element at 8 points, 10.9 KB at 20; allocated by the system when it is
+ * finish. The first keeps records of up to 1 GiB on the device (5.6 KB an
+ * element at 8 points, 14.1 KB at 20; allocated by the system when it is
  * made or its element changes). sbk_set_local_iteration sets what sbk_element_batch
  * uses and what new systems start with. */
 #define SBK_LOCAL_PHASES 0
