@@ -52,9 +52,9 @@ METRIC = "Hex8 tangent+residual+assembly elem/s (FP64)"
 # DRAM bytes (read + write) per element of one evaluation's K1: ncu's
 # dram__bytes_read.sum + dram__bytes_write.sum summed over its launches in one
 # evaluation of the same construction at 80,000 elements (200 x 200 x 2):
-# 1.71 GB (the tile kernel 0.63, the condensation 0.69, the single kernel's
-# share 0.38); the traffic grows with the elements.
-K1_DRAM_BYTES_PER_ELEMENT = 1.706e9 / 80000
+# 1.36 GB (the tile kernel 0.65, the condensation 0.72); the traffic grows with
+# the elements.
+K1_DRAM_BYTES_PER_ELEMENT = (0.649201920e9 + 0.715312384e9) / 80000
 
 
 def record_chunks(ne):
@@ -66,9 +66,9 @@ def record_chunks(ne):
 # The single kernel (--local-iteration single): 0.69 + 5.28 GB in one launch
 # at 80,000 elements.
 K1_SINGLE_DRAM_BYTES_PER_ELEMENT = (0.692594688e9 + 5.275133e9) / 80000
-# The same for the standard Hex8 kernel: 0.192 GB read + 1.610 GB written in
-# one launch at 80,000 elements.
-K1S_DRAM_BYTES_PER_ELEMENT = (0.191949568e9 + 1.610487e9) / 80000
+# The same for the standard Hex8: 0.67 GB by its points' kernel, 0.77 GB by
+# its tangents'.
+K1S_DRAM_BYTES_PER_ELEMENT = (0.672582400e9 + 0.771357184e9) / 80000
 # DRAM bytes per block entry of one free-free gather (assemble): the same ncu
 # metrics over one launch on the 200 x 200 x 2 sheet's block, 271.0 MB read +
 # 139.0 MB written for 22,528,485 entries.

@@ -25,7 +25,7 @@
 //
 // Why: as one launch per stage over the whole mesh (130 launches) the stages
 // handed each other 207 KB per element through DRAM, and a mesh of a few
-// thousand elements spent its time on launches. On chip an element moves 21
+// thousand elements spent its time on launches. On chip an element moves 17
 // KB, its state, K* and the condensation's record among them. What bounds a
 // stage is the latency of one warp's chain (a stage takes nearly as long for
 // one warp as for eight) and the fetch of its instructions: with two blocks
@@ -34,9 +34,9 @@
 // block, and code that is in the kernel once.
 //
 // Measured (B200; an evaluation's element kernels before and after, all of
-// them): 80 J2 elements 543 -> 92 us, 3,200 626 -> 170 us; Hill48 + two-term
-// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.47 ms, 22,350 of
-// them 32.4 -> 2.8 ms; 1,000,000 of the 2 x 2 x 2 rule 82.1 -> 50.3 ms.
+// them): 80 J2 elements 543 -> 91 us, 3,200 626 -> 166 us; Hill48 + two-term
+// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.46 ms, 22,350 of
+// them 32.4 -> 2.8 ms; 1,000,000 of the 2 x 2 x 2 rule 82.1 -> 49.6 ms.
 //
 // The algorithm and its constants are element_kernel's (sbk_element.cu),
 // which cites the reference.
