@@ -170,8 +170,8 @@ int sbk_system_set_values_buffer(sbk_system* sys, double* values_dev);
 
 /* Launch shape of the element kernel: elements per thread block. 0, the
  * default: a tile of as many elements as the block has threads for their
- * points (32 at 8 points, 12 at 20), fewer on a mesh too small to fill the
- * GPU with full tiles; for the single kernel 16 for rules of up to 8 points
+ * points (32 at 8 points, 12 at 20), or fewer, so that the tiles fill the
+ * GPU a whole number of times; for the single kernel 16 for rules of up to 8 points
  * - four warps - and 8 for larger rules - eight warps. At most what 227 KB of
  * shared memory and 256 threads hold; the batch autotuner sets it. */
 int sbk_system_set_elements_per_block(sbk_system* sys, int elements_per_block);

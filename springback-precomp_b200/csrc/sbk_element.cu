@@ -1683,15 +1683,18 @@ namespace {
 template <class After>
 int run_tiles(const Params& p, TileArgs a, const TileScratch& s, int elements_per_block, cudaStream_t stream,
               After after) {
-  // A full tile per block once the mesh has that many elements; below, the
-  // elements spread evenly over the blocks that are resident at once.
+  // As many elements a tile as make the waves of tiles full ones: n elements
+  // in ceil(n / (148 most)) waves. Full tiles leave a last wave of a few that
+  // takes as long as the others: 2,304 elements of 20 points, 379 us as 192
+  // tiles of 12, 327 us as 288 of 8; 8,192 of 8 points 190 and 178 us. From
+  // five waves on there is no difference (23,086 of 8 points: 975 us).
   const int most = tile_most(p.nq);
-  const int64_t even = (a.ne + kTileBlocks - 1) / kTileBlocks;
-  a.elements = elements_per_block > 0 ? elements_per_block : (int)(even < most ? even : most);
-  if (a.elements > most) a.elements = most;
   const int64_t chunk = tile_chunk(p.nq);
   for (a.begin = 0; a.begin < a.ne; a.begin += chunk) {
     a.end = a.ne - a.begin < chunk ? a.ne : a.begin + chunk;
+    const int64_t n = a.end - a.begin, waves = (n + kTileBlocks * most - 1) / (kTileBlocks * most);
+    a.elements = elements_per_block > 0 ? elements_per_block : (int)((n + kTileBlocks * waves - 1) / (kTileBlocks * waves));
+    if (a.elements > most) a.elements = most;
     a.num_tiles = (int)((a.end - a.begin + a.elements - 1) / a.elements);
     const unsigned grid = (unsigned)(a.num_tiles < kTileBlocks ? a.num_tiles : kTileBlocks);
     cudaError_t err = cudaMemsetAsync(s.counts, 0, (a.begin == 0 ? 2 : 1) * sizeof(int32_t), stream);

@@ -35,7 +35,7 @@
 //
 // Measured (B200; an evaluation's element kernels before and after, all of
 // them): 80 J2 elements 543 -> 91 us, 3,200 626 -> 166 us; Hill48 + two-term
-// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.46 ms, 22,350 of
+// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.41 ms, 22,350 of
 // them 32.4 -> 2.8 ms; 1,000,000 of the 2 x 2 x 2 rule 82.1 -> 49.6 ms.
 //
 // The algorithm and its constants are element_kernel's (sbk_element.cu),
