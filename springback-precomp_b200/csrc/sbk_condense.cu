@@ -10,21 +10,22 @@
 // the limit. The 33rd degree of freedom and the stress (f_u) would each open
 // a tile of one column or row: they go as FMAs, four lanes an entry. Measured
 // on 1,000,000 elements (2 x 2 x 2 points, non-symmetric): 17.8 ms as FMAs of
-// 8 lanes an element, 12.4 ms all in tiles, 11.4 ms so; the tensor
-// instructions alone are 5.5 ms of it. Four blocks an SM (spilling at 128
-// registers) take 12.0 ms, two points unrolled 12.1.
+// 8 lanes an element, 12.4 ms all in tiles, 11.4 ms so, 9.2 ms with the
+// table filled straight through (sbk_point_table.cuh); the tensor instructions
+// alone are 5.5 ms of it. Four blocks an SM (spilling at 128 registers) or two
+// points unrolled took 5 % longer.
 #include <cuda_runtime.h>
 
 #include "sbk_element_math.cuh"
+#include "sbk_point_table.cuh"
 #include "sbk_tile.h"
 
 namespace sbk {
 namespace {
 
 constexpr int kWarps = 4;
-// Per point of the gradient table: 11 gradients of five entries (x y z x y)
-// and the rows of F alike, so that the cyclic components t, t + 1, t + 2 of a
-// lane are three consecutive entries; three zeros.
+// Per point of the table (sbk_point_table.cuh): 11 gradients, the rows of F,
+// three zeros.
 constexpr int kTabF = 55, kTabZero = 70, kTab = 73;
 constexpr int kKua = 0;    // 24 x 10: K_ua and f_u (over the record's points)
 constexpr int kC = 240;    // 9 x 25: K_au and r_a, then their solutions
@@ -101,34 +102,8 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
   for (int q0 = 0; q0 < nq; q0 += 8) {
     const int count = min(8, nq - q0);
     __syncwarp();
-    for (int idx = lane; idx < count * 45; idx += 32) {
-      const int qq = idx / 45, c = idx - 45 * qq, q = q0 + qq;
-      double* T = tab + qq * kTab;
-      double v = 0.0;
-      int at;
-      if (c < 33) {
-        const int n = c / 3, i = c - 3 * n;
-        if (n < 8) {
-          const double sx = ((n + 1) >> 1) & 1 ? 1.0 : -1.0, sy = (n >> 1) & 1 ? 1.0 : -1.0, sz = n >> 2 ? 1.0 : -1.0;
-          const double fx = 1.0 + p.qp[q][0] * sx, fy = 1.0 + p.qp[q][1] * sy, fz = 1.0 + p.qp[q][2] * sz;
-          const double* ji = rec + (kCondGeo + i) * nq + q;
-          v = 0.125 * (sx * fy * fz * ji[0] + sy * fx * fz * ji[3 * nq] + sz * fx * fy * ji[6 * nq]);
-        } else {
-          v = rec[(kCondGeo + 9) * nq + q] * (-2.0 * p.qp[q][n - 8]) * own[kCondJ0 + (n - 8) * 3 + i];
-        }
-        at = 5 * n + i;
-        T[at] = v;
-        if (i < 2) T[at + 3] = v;
-      } else if (c < 42) {
-        const int f = c - 33, i = f % 3;
-        v = (small ? 0.0 : rec[(kCondH + f) * nq + q]) + (f % 4 == 0 ? 1.0 : 0.0);
-        at = kTabF + 5 * (f / 3) + i;
-        T[at] = v;
-        if (i < 2) T[at + 3] = v;
-      } else {
-        T[kTabZero + c - 42] = 0.0;
-      }
-    }
+    if (g < count)
+      point_table<true>(p, q0 + g, t, small, rec + q0 + g, nq, own + kCondJ0, tab + g * kTab, kTabF, kTabZero);
     __syncwarp();
 #pragma unroll 1
     for (int qq = 0; qq < count; ++qq) {

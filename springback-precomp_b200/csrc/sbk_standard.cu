@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "sbk_element.h"
+#include "sbk_point_table.cuh"
 #include "sbk_tile_point.cuh"
 
 namespace sbk {
@@ -282,8 +283,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 // ---- force and tangent ---------------------------------------------------------
 
 constexpr int kWarps = 4;
-// Per point of the table: eight gradients and F's rows of five entries (x y z
-// x y), three zeros (as in the condensation).
+// Per point of the table (sbk_point_table.cuh): eight gradients, the rows of
+// F, three zeros.
 constexpr int kTabF = 40, kTabZero = 55, kTab = 58;
 constexpr int kExtra = 8 * kTab + 64;
 
@@ -358,26 +359,8 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
       const int count = min(8, nq - q0);
       if (!AVERAGED || nq > 8 || pass == 0) {
         __syncwarp();
-        for (int idx = lane; idx < count * 36; idx += 32) {
-          const int qq = idx / 36, c = idx - 36 * qq, q = q0 + qq;
-          double* T = tab + qq * kTab;
-          if (c < 24) {
-            const int n = c / 3, i = c - 3 * n;
-            const double sx = ((n + 1) >> 1) & 1 ? 1.0 : -1.0, sy = (n >> 1) & 1 ? 1.0 : -1.0, sz = n >> 2 ? 1.0 : -1.0;
-            const double fx = 1.0 + p.qp[q][0] * sx, fy = 1.0 + p.qp[q][1] * sy, fz = 1.0 + p.qp[q][2] * sz;
-            const double* ji = rec + (kCondGeo + i) * nq + q;
-            const double v = 0.125 * (sx * fy * fz * ji[0] + sy * fx * fz * ji[3 * nq] + sz * fx * fy * ji[6 * nq]);
-            T[5 * n + i] = v;
-            if (i < 2) T[5 * n + i + 3] = v;
-          } else if (c < 33) {
-            const int f = c - 24, i = f % 3;
-            const double v = (small ? 0.0 : rec[(kCondH + f) * nq + q]) + (f % 4 == 0 ? 1.0 : 0.0);
-            T[kTabF + 5 * (f / 3) + i] = v;
-            if (i < 2) T[kTabF + 5 * (f / 3) + i + 3] = v;
-          } else {
-            T[kTabZero + c - 33] = 0.0;
-          }
-        }
+        if (g < count)
+          point_table<false>(p, q0 + g, t, small, rec + q0 + g, nq, nullptr, tab + g * kTab, kTabF, kTabZero);
         __syncwarp();
       }
 #pragma unroll 1
