@@ -15,7 +15,7 @@
 //
 // Measured (7,200 J2 elements with mean dilatation): 479 us for the element
 // kernel that had a group of lanes and 12 KB of shared memory an element, and
-// 49 us for its schedule; 55 + 73 us so.
+// 49 us for its schedule; 51 + 64 us so.
 #include <cuda_runtime.h>
 
 #include "sbk_element.h"

@@ -55,7 +55,7 @@ namespace sbk {
 constexpr int kRecH = 0;       // displacement gradient 9
 constexpr int kRecM = 9;       // material block 36
 constexpr int kRecS = 45;      // stress 6
-constexpr int kRecHmax = 51;   // largest |H|, then the point's energy
+constexpr int kRecHmax = 51;   // largest |H|, then (map) its share of the floor, then the point's energy
 constexpr int kRecW = 52;      // w det J
 constexpr int kRecL = 53;      // axes 9, mu 3, first 6
 constexpr int kRecStrain = 71;
@@ -216,6 +216,7 @@ struct Tile {
   __device__ __forceinline__ void map(int pt) {
     const PointRecord r = point(pt);
     const bool elastic = (flag[pt] & 3) == 0;
+    double mmax = 0.0;  // the block's largest entry
     if (p.kinematics == SBK_FINITE_LOGARITHMIC) {
       LogKin L;
 #pragma unroll
@@ -224,13 +225,19 @@ struct Tile {
       for (int i = 0; i < 3; ++i) L.mu[i] = r.get(kRecL + 9 + i);
 #pragma unroll
       for (int i = 0; i < 6; ++i) L.first[i] = r.get(kRecL + 12 + i);
-      spectral_map(p, L, elastic, r, kRecS, kRecM);
-    } else if (elastic) {
-      double C[36];
-      elastic_C(p, C);
+      mmax = spectral_map(p, L, elastic, r, kRecS, kRecM);
+    } else {
+      if (elastic) {
+        double C[36];
+        elastic_C(p, C);
 #pragma unroll
-      for (int i = 0; i < 36; ++i) r.put(kRecM + i, C[i]);
+        for (int i = 0; i < 36; ++i) r.put(kRecM + i, C[i]);
+      }
+#pragma unroll 6
+      for (int i = 0; i < 36; ++i) mmax = fmax(mmax, fabs(r.get(kRecM + i)));
     }
+    const double hmax = r.get(kRecHmax);
+    r.put(kRecHmax, r.get(kRecW) * mmax * hmax * (1.0 + hmax));
   }
 
   // Rows 3m..3m+2 of K_aa and r_a, and the scale and floor sums of mode m:
@@ -256,15 +263,12 @@ struct Tile {
       double F[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) F[i] = (small ? 0.0 : r.get(kRecH + i)) + ((i % 4) == 0 ? 1.0 : 0.0);
-      double W[3][6], mmax = 0.0;
+      double W[3][6];
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
         double col[6];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-          col[i] = r.get(kRecM + i * 6 + c);
-          mmax = fmax(mmax, fabs(col[i]));
-        }
+        for (int i = 0; i < 6; ++i) col[i] = r.get(kRecM + i * 6 + c);
         W[0][c] = w * (g[0] * col[0] + g[1] * col[3] + g[2] * col[5]);
         W[1][c] = w * (g[0] * col[3] + g[1] * col[1] + g[2] * col[4]);
         W[2][c] = w * (g[0] * col[5] + g[1] * col[4] + g[2] * col[2]);
@@ -282,7 +286,7 @@ struct Tile {
 #pragma unroll
         for (int i = 0; i < 3; ++i) gn[n][i] = f * E.jinv0[n * 3 + i];
       }
-      const double hmax = r.get(kRecHmax), floor_w = w * mmax * hmax * (1.0 + hmax);
+      const double floor_w = r.get(kRecHmax);
 #pragma unroll
       for (int kk = 0; kk < 3; ++kk) {
         double Uk[6];

@@ -264,8 +264,8 @@ __device__ __forceinline__ double spectral_second(const LogKin& L, int k, int j,
 // point's record and passes through row by row and column by column: 36
 // values in registers would leave no room for more warps, and unrolled they
 // are 20 KB of code that every tile fetches each round.
-__device__ __forceinline__ void spectral_map(const Params& p, const LogKin& L, bool elastic, const PointRecord& rec,
-                                             int fS, int fM) {
+__device__ __forceinline__ double spectral_map(const Params& p, const LogKin& L, bool elastic, const PointRecord& rec,
+                                               int fS, int fM) {
   double tp[6];
   {
     double t[6];
@@ -323,6 +323,7 @@ __device__ __forceinline__ void spectral_map(const Params& p, const LogKin& L, b
 #pragma unroll
     for (int i = 0; i < 6; ++i) rec.put(fM + i * 6 + j, col[i]);
   }
+  double top = 0.0;
 #pragma unroll 1
   for (int i = 0; i < 6; ++i) {
     double row[6], r[6];
@@ -330,7 +331,10 @@ __device__ __forceinline__ void spectral_map(const Params& p, const LogKin& L, b
     for (int j = 0; j < 6; ++j) row[j] = rec.get(fM + i * 6 + j);
     rotate_out(L.q, row, r);
 #pragma unroll
-    for (int j = 0; j < 6; ++j) rec.put(fM + i * 6 + j, r[j]);
+    for (int j = 0; j < 6; ++j) {
+      rec.put(fM + i * 6 + j, r[j]);
+      top = fmax(top, fabs(r[j]));
+    }
   }
   double t[6];
 #pragma unroll
@@ -338,6 +342,7 @@ __device__ __forceinline__ void spectral_map(const Params& p, const LogKin& L, b
   rotate_out(L.q, tp, t);
 #pragma unroll
   for (int i = 0; i < 6; ++i) rec.put(fS + i, t[i]);
+  return top;
 }
 
 // ---- the trial state ------------------------------------------------------------
