@@ -11,8 +11,8 @@
 //             strain, the trial state; the points that yield are listed;
 //   returns   a thread a listed point: the closest-point (or radial) return;
 //   map       a thread a point: the logarithmic map of stress and tangent;
-//   sums      a thread a (point, mode): the mode's rows of K_aa, r_a and the
-//             scale and floor sums, over the points by shuffles;
+//   sums      four lanes a (mode, element): the mode's rows of K_aa, r_a and
+//             the scale and floor sums, over the points, then by shuffles;
 //   control   16 lanes an element: acceptance of the trial, the pivoted LU
 //             of K_aa with a row per lane in registers, Newton's direction,
 //             the definiteness test.
@@ -34,9 +34,9 @@
 // block, and code that is in the kernel once.
 //
 // Measured (B200; an evaluation's element kernels before and after, all of
-// them): 80 J2 elements 543 -> 91 us, 3,200 626 -> 166 us; Hill48 + two-term
-// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.41 ms, 22,350 of
-// them 32.4 -> 2.8 ms; 1,000,000 of the 2 x 2 x 2 rule 82.1 -> 49.6 ms.
+// them): 80 J2 elements 543 -> 88 us, 3,200 626 -> 157 us; Hill48 + two-term
+// Chaboche: 2,304 elements of the 2 x 2 x 5 rule 3.39 -> 0.37 ms, 22,350 of
+// them 32.4 -> 2.5 ms; 1,000,000 of the 2 x 2 x 2 rule 82.1 -> 45.5 ms.
 //
 // The algorithm and its constants are element_kernel's (sbk_element.cu),
 // which cites the reference.
@@ -89,6 +89,10 @@ __device__ __forceinline__ double pick9(const double a[9], int k) {
   return v;
 }
 constexpr unsigned kAll = 0xffffffffu;
+// Lanes of a (mode, element) in sums. Eight split 20 points into 3 each, and 12
+// elements' 288 lanes into two passes of the block; four take 5 each in one:
+// 2.09 -> 2.01 ms for 22,350 elements. At 8 points there is no difference.
+constexpr int kSumLanes = 4;
 
 template <int NT>
 struct Tile {
@@ -241,16 +245,16 @@ struct Tile {
   }
 
   // Rows 3m..3m+2 of K_aa and r_a, and the scale and floor sums of mode m:
-  // lane l of eight sums the points l, l + 8, ..., the eight then by a
-  // reduce-scatter. V(k, l, n) as in vtensor.
+  // lane l of kSumLanes sums the points l, l + kSumLanes, ..., the lanes
+  // then by a reduce-scatter. V(k, l, n) as in vtensor.
   __device__ __forceinline__ void sums(int k, int m, int lane, bool live) {
     TileElement& E = el[k];
-    double acc[40];
+    double acc[36];
 #pragma unroll
-    for (int i = 0; i < 40; ++i) acc[i] = 0.0;
+    for (int i = 0; i < 36; ++i) acc[i] = 0.0;
     const bool small = p.kinematics == SBK_SMALL_STRAIN;
 #pragma unroll 1
-    for (int q = live ? lane : nq; q < nq; q += 8) {
+    for (int q = live ? lane : nq; q < nq; q += kSumLanes) {
       const int pt = k * nq + q;
       const PointRecord r = point(pt);
       const double w = r.get(kRecW), ratio = geo[9 * np + pt];
@@ -323,12 +327,12 @@ struct Tile {
       }
     }
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      double v[8];
+    for (int c = 0; c < 36 / kSumLanes; ++c) {
+      double v[kSumLanes];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = acc[c * 8 + i];
-      const double y = reduce_scatter<8>(v, lane, 0xffffffffu);
-      const int i = c * 8 + lane;
+      for (int i = 0; i < kSumLanes; ++i) v[i] = acc[c * kSumLanes + i];
+      const double y = reduce_scatter<kSumLanes>(v, lane, 0xffffffffu);
+      const int i = c * kSumLanes + lane;
       if (!live) continue;
       if (i < 27) E.kc[(3 * m) * 9 + i] = y;
       else if (i < 30) E.r[3 * m + i - 27] = y;
@@ -655,12 +659,12 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSm)
         if (T.el[k].fail == 0x7fffffff) T.map(k * nq + i - j * nq);
       }
       __syncthreads();
-      // Eight lanes a (mode, element).
+      // Four lanes a (mode, element).
 #pragma unroll 1
-      for (int i = tid; i - lane < n * 24; i += kTileThreads) {
-        const bool task = i < n * 24;
-        const int j = task ? i >> 3 : 0, m = j / n, k = active[side][j - m * n];
-        T.sums(k, m, i & 7, task && T.el[k].fail == 0x7fffffff);
+      for (int i = tid; i - lane < n * 3 * kSumLanes; i += kTileThreads) {
+        const bool task = i < n * 3 * kSumLanes;
+        const int j = task ? i / kSumLanes : 0, m = j / n, k = active[side][j - m * n];
+        T.sums(k, m, i % kSumLanes, task && T.el[k].fail == 0x7fffffff);
       }
       __syncthreads();
 #pragma unroll 1
