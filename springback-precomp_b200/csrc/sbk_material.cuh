@@ -478,7 +478,7 @@ __device__ __forceinline__ void general_trial(const Params& p, const double stra
     for (int j = 0; j < 6; ++j) s += p.P[i * 6 + j] * T.xi_tr[j];
     q += T.xi_tr[i] * s;
   }
-  T.eq_trial = sqrt(fmax(q, 0.0));
+  T.eq_trial = sqrt(q < 0.0 ? 0.0 : q);  // a NaN stays one (fmax would drop it): the return fails on it
   T.f_trial = T.eq_trial - T.sy_n;
 }
 

@@ -362,11 +362,17 @@ struct Tile {
       floors = fmax(floors, __shfl_xor_sync(kAll, floors, o, 16));
     }
     full = sqrt(full);
+    // fmax drops a NaN, the sum keeps it: a residual that is not a number
+    // is no residual of 0 (the lanes beyond the rows), nor an infinite one
+    // within an infinite bound.
+    if (isnan(full)) largest = full;
+    const bool finite = isfinite(largest);
     const double bound = kLocalTolerance * scale + kLocalRoundOff * floors;
     // The full Newton step, accepted when it reduces the residual enough or
     // meets the tolerance; everything else is search_after's.
     const bool evaluated = fail == 0x7fffffff;
-    const bool reduced = evaluated && (full <= kFullStepReduction * E.res || largest <= bound);
+    const bool met = finite && largest <= bound;
+    const bool reduced = evaluated && finite && (full <= kFullStepReduction * E.res || met);
     int out = -1;
     bool go = live && (first ? evaluated : E.stage == kStageNewton && reduced);
     if (live && first && !evaluated) out = (fail & 0xff) << 8;
@@ -374,7 +380,7 @@ struct Tile {
     if (__any_sync(kAll, look)) {
       int got = 0;
       if (look && lane == 0)
-        got = search_after(E, E.search, evaluated, full, largest <= bound, full <= kFullStepReduction * E.res);
+        got = search_after(E, E.search, evaluated, full, met, full <= kFullStepReduction * E.res);
       got = __shfl_sync(kAll, got, 0, 16);
       __syncwarp();
       if (look) {
@@ -396,7 +402,7 @@ struct Tile {
     __syncwarp();
     if (go && row) E.alpha[lane] = E.at[lane];
     double myinv = 0.0, big_pivot = 0.0, small_pivot = 1.0e308;
-    bool positive = true;
+    bool positive = true, pivots = true;  // a NaN is neither
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
       const double d = __shfl_sync(kAll, A[s], s, 16);
@@ -409,23 +415,24 @@ struct Tile {
       b -= l * __shfl_sync(kAll, b, s, 16);
       if (lane > s) A[s] = l;
       if (lane == s) myinv = inv;
-      positive = positive && !(d <= 0.0);
+      pivots = pivots && d > 0.0;
     }
-    if (!symmetric) {
-      positive = true;
+    if (symmetric) {
+      positive = pivots;
+    } else {
 #pragma unroll
       for (int s = 0; s < 9; ++s) {
         const double d = __shfl_sync(kAll, sym[s], s, 16);
-        positive = positive && !(d <= 0.0);
+        positive = positive && d > 0.0;
         const double l = lane > s ? sym[s] * (1.0 / d) : 0.0;
 #pragma unroll
         for (int j = s + 1; j < 9; ++j) sym[j] -= l * __shfl_sync(kAll, sym[j], s, 16);
       }
     }
-    const bool converged = largest <= bound || largest == 0.0;
+    const bool converged = met || largest == 0.0;
     // Definite and far from singular: no pivot search is needed. Anything
     // else takes the complete pivoting and its rank test.
-    const bool pivot = go && !(positive && small_pivot > 1.0e-10 * big_pivot);
+    const bool pivot = go && !(positive && pivots && small_pivot > 1.0e-10 * big_pivot);
     int status = -1;
     if (__any_sync(kAll, pivot)) status = pivoted(E, pivot, r, converged, lane);
     if (go) {
@@ -440,7 +447,7 @@ struct Tile {
         }
         out = 1;
       } else {
-        out = E.iterations == kMaxLocal || !isfinite(largest) ? SBK_EL_LOCAL_NO_CONVERGE << 8 : (positive ? 0 : 2);
+        out = E.iterations == kMaxLocal || !finite ? SBK_EL_LOCAL_NO_CONVERGE << 8 : (positive ? 0 : 2);
       }
     }
     const bool on = go && out == 0;

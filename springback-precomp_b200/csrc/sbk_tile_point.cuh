@@ -409,7 +409,7 @@ __device__ __forceinline__ void point_trial(const Params& p, const double strain
       for (int j = 0; j < 6; ++j) v += p.P[i * 6 + j] * T.xi[j];
       q += T.xi[i] * v;
     }
-    T.eq = sqrt(fmax(q, 0.0));
+    T.eq = sqrt(q < 0.0 ? 0.0 : q);  // a NaN stays one (fmax would drop it): the return fails on it
   }
   T.f = T.eq - T.sy;
 }
