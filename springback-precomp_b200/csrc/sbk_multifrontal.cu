@@ -21,8 +21,8 @@
 // and the solves walk the same levels with a block a front. What bounds it is
 // the chain of levels and panels, some hundred launches of a few microseconds
 // for a sheet of 13,689 rows. Measured there (41 x 41 x 3 nodes, clamped):
-// factorisation and solve 44.7 ms with the level-scheduled sparse Cholesky of
-// the library, 1.5 ms so.
+// factorisation and one solve 44.7 ms with the level-scheduled sparse Cholesky
+// of the library, 1.5 ms so.
 #include "sbk_multifrontal.h"
 
 #include <algorithm>
