@@ -18,6 +18,7 @@
 
 #include "sbk_element_math.cuh"
 #include "sbk_point_table.cuh"
+#include "sbk_smem.h"
 #include "sbk_tile.h"
 
 namespace sbk {
@@ -282,16 +283,11 @@ __global__ void __launch_bounds__(kWarps * 32, SYM || !TANGENT ? 4 : 3)
 
 template <bool SYM, bool TANGENT>
 int launch(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream) {
-  static size_t raised[64] = {};
+  static SmemLimit limit;
   const size_t smem = (size_t)kWarps * warp_doubles(p.nq) * sizeof(double);
-  int dev = 0;
-  cudaGetDevice(&dev);
   auto kern = condense_kernel<SYM, TANGENT>;
-  if (dev < 0 || dev >= 64 || raised[dev] < smem) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    if (dev >= 0 && dev < 64) raised[dev] = smem;
-  }
+  const cudaError_t err = limit.allow(kern);
+  if (err != cudaSuccess) return (int)err;
   const int64_t n = a.end - a.begin;
   kern<<<(unsigned)((n + kWarps - 1) / kWarps), kWarps * 32, smem, stream>>>(p, a.begin, a.end, s.cond, a.code,
                                                                              a.force, a.tangent);

@@ -25,6 +25,7 @@
 #include "sbk_element.h"
 #include "sbk_element_math.cuh"
 #include "sbk_material.cuh"
+#include "sbk_smem.h"
 #include "sbk_tile.h"
 
 namespace sbk {
@@ -1599,17 +1600,9 @@ int launch_g(const Params& p, int64_t ne, const double* coords, const int32_t* c
   const int64_t blocks = (ne + epb - 1) / epb;
   if (blocks == 0) return 0;
   auto kern = element_kernel<G>;
-  // The shared-memory limit is raised once per device and size, so that a
-  // launch inside a stream capture (a CUDA graph of an evaluation) makes no
-  // attribute call.
-  static size_t raised[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || raised[dev] < smem) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    if (dev >= 0 && dev < 64) raised[dev] = smem;
-  }
+  static SmemLimit limit;
+  const cudaError_t err = limit.allow(kern);
+  if (err != cudaSuccess) return (int)err;
   kern<<<(unsigned)blocks, threads, smem, stream>>>(p, ne, batch, coords, conn, u, state, alpha_n, want_tangent,
                                                      force, tangent, energy, trial, alpha_out, yield, iterations,
                                                      code, first_failure, order);
@@ -1619,20 +1612,6 @@ int launch_g(const Params& p, int64_t ne, const double* coords, const int32_t* c
 }  // namespace
 
 namespace {
-
-// The shared-memory limit of a kernel raised once per device, so that a
-// launch inside a stream capture makes no attribute call.
-template <class K>
-int raise_smem(K kern, size_t smem, size_t* raised) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || raised[dev] < smem) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    if (dev >= 0 && dev < 64) raised[dev] = smem;
-  }
-  return 0;
-}
 
 // Elements of a full tile: the points of a block's threads, at most
 // kTileMostElements.
@@ -1715,11 +1694,11 @@ int run_tiles(const Params& p, TileArgs a, const TileScratch& s, int elements_pe
 // The elements handed on, by a list kernel that starts each again with
 // `record` bytes of shared memory an element (one block of it per SM).
 template <class K, class... A>
-int run_list(K kern, int64_t ne, int group, size_t record, size_t* raised, cudaStream_t stream, const A&... args) {
+int run_list(K kern, int64_t ne, int group, size_t record, SmemLimit& limit, cudaStream_t stream, const A&... args) {
   const int epb = group == 8 ? 16 : 8;
   const size_t smem = record * epb;
-  const int bad = raise_smem(kern, smem, raised);
-  if (bad) return bad;
+  const cudaError_t err = limit.allow(kern);
+  if (err != cudaSuccess) return (int)err;
   const int64_t need = (ne + epb - 1) / epb;
   kern<<<(unsigned)(need < 148 * 2 ? need : 148 * 2), epb * group, smem, stream>>>(args...);
   return (int)cudaGetLastError();
@@ -1739,12 +1718,12 @@ int launch_elements_tile(const Params& p, int64_t ne, const double* coords, cons
     return p.element == 1 ? 0 : launch_condense(p, at, s, stream);
   });
   if (rc || p.element == 1) return rc;
-  static size_t raised[2][64] = {};
+  static SmemLimit limit[2];
   if (p.nq <= 8)
-    return run_list(element_list_kernel<8>, ne, 8, sizeof(ElemShared<8>), raised[0], stream, p, ne, batch, coords,
+    return run_list(element_list_kernel<8>, ne, 8, sizeof(ElemShared<8>), limit[0], stream, p, ne, batch, coords,
                     conn, u, state, alpha_n, want_tangent, force, tangent, energy, trial, alpha_out, yield,
                     iterations, code, first_failure, s.fallback, s.counts + 1);
-  return run_list(element_list_kernel<32>, ne, 32, sizeof(ElemShared<32>), raised[1], stream, p, ne, batch, coords,
+  return run_list(element_list_kernel<32>, ne, 32, sizeof(ElemShared<32>), limit[1], stream, p, ne, batch, coords,
                   conn, u, state, alpha_n, want_tangent, force, tangent, energy, trial, alpha_out, yield, iterations,
                   code, first_failure, s.fallback, s.counts + 1);
 }
@@ -1759,11 +1738,11 @@ int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t*
   const int rc = run_tiles(p, a, s, elements_per_block, stream,
                            [&](const TileArgs& at) { return launch_vjp_tile(p, at, s, lambda, out, stream); });
   if (rc) return rc;
-  static size_t raised[2][64] = {};
+  static SmemLimit limit[2];
   if (p.nq <= 8)
-    return run_list(vjp_kernel<8>, ne, 8, sizeof(ElemShared<8>), raised[0], stream, p, ne, coords, conn, u, state,
+    return run_list(vjp_kernel<8>, ne, 8, sizeof(ElemShared<8>), limit[0], stream, p, ne, coords, conn, u, state,
                     alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
-  return run_list(vjp_kernel<32>, ne, 32, sizeof(ElemShared<32>), raised[1], stream, p, ne, coords, conn, u, state,
+  return run_list(vjp_kernel<32>, ne, 32, sizeof(ElemShared<32>), limit[1], stream, p, ne, coords, conn, u, state,
                   alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
 }
 

@@ -20,6 +20,7 @@
 
 #include "sbk_element.h"
 #include "sbk_point_table.cuh"
+#include "sbk_smem.h"
 #include "sbk_tile_point.cuh"
 
 namespace sbk {
@@ -465,35 +466,23 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   for (int i = 0; i < 18; ++i) out[lane + 32 * i] = x[lane + 32 * i];
 }
 
-template <class K>
-int raise_smem(K kern, size_t smem, size_t* raised) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || raised[dev] < smem) {
-    const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    if (dev >= 0 && dev < 64) raised[dev] = smem;
-  }
-  return 0;
-}
-
 template <int NT>
 int launch_points(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream) {
-  static size_t raised[64] = {};
+  static SmemLimit limit;
   const size_t np = (size_t)(a.elements * p.nq) | 1;
   const size_t smem = (kRec * np + 48u * a.elements) * sizeof(double);
-  const int rc = raise_smem(standard_points_kernel<NT>, smem, raised);
-  if (rc) return rc;
+  const cudaError_t err = limit.allow(standard_points_kernel<NT>);
+  if (err != cudaSuccess) return (int)err;
   standard_points_kernel<NT><<<(unsigned)a.num_tiles, kThreads, smem, stream>>>(p, a, s.cond);
   return (int)cudaGetLastError();
 }
 
 template <bool SYM, bool AVERAGED>
 int launch_tangent(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream) {
-  static size_t raised[64] = {};
+  static SmemLimit limit;
   const size_t smem = (size_t)kWarps * warp_doubles(p.nq) * sizeof(double);
-  const int rc = raise_smem(standard_tangent_kernel<SYM, AVERAGED>, smem, raised);
-  if (rc) return rc;
+  const cudaError_t err = limit.allow(standard_tangent_kernel<SYM, AVERAGED>);
+  if (err != cudaSuccess) return (int)err;
   const int64_t n = a.end - a.begin;
   standard_tangent_kernel<SYM, AVERAGED><<<(unsigned)((n + kWarps - 1) / kWarps), kWarps * 32, smem, stream>>>(
       p, a.begin, a.end, s.cond, a.code, a.force, a.tangent, a.want_tangent);

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "sbk_element.h"
+#include "sbk_smem.h"
 #include "sbk_tile_point.cuh"
 
 namespace sbk {
@@ -269,27 +270,30 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
+template <int NT>
+int launch(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u, const double* state,
+           const double* alpha_n, double* out, int32_t* code, int32_t* first_failure, cudaStream_t stream) {
+  static SmemLimit limit;
+  const cudaError_t err = limit.allow(stress_kernel<NT>);
+  if (err != cudaSuccess) return (int)err;
+  const int elements = kThreads / p.nq < kElements ? kThreads / p.nq : kElements;
+  const size_t np = (size_t)(elements * p.nq) | 1;
+  const size_t smem = (kOut * np + 57u * elements) * sizeof(double);
+  const unsigned grid = (unsigned)((ne + elements - 1) / elements);
+  stress_kernel<NT><<<grid, kThreads, smem, stream>>>(p, ne, elements, coords, conn, u, state, alpha_n, out, code,
+                                                      first_failure);
+  return (int)cudaGetLastError();
+}
+
 }  // namespace
 
 int launch_stress(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,
                   const double* state, const double* alpha_n, double* out, int32_t* code, int32_t* first_failure,
                   cudaStream_t stream) {
   if (ne <= 0) return 0;
-  const int elements = kThreads / p.nq < kElements ? kThreads / p.nq : kElements;
-  const size_t np = (size_t)(elements * p.nq) | 1;
-  const size_t smem = (kOut * np + 57u * elements) * sizeof(double);
-  const unsigned grid = (unsigned)((ne + elements - 1) / elements);
-  auto run = [&](auto kern) {
-    const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    kern<<<grid, kThreads, smem, stream>>>(p, ne, elements, coords, conn, u, state, alpha_n, out, code, first_failure);
-    return (int)cudaGetLastError();
-  };
-  if (!p.general) return run(stress_kernel<-1>);
-  if (p.nterms == 0) return run(stress_kernel<0>);
-  if (p.nterms == 1) return run(stress_kernel<1>);
-  if (p.nterms == 2) return run(stress_kernel<2>);
-  return run(stress_kernel<4>);
+  const auto run = !p.general ? launch<-1>
+                              : (p.nterms == 0 ? launch<0> : (p.nterms == 1 ? launch<1> : (p.nterms == 2 ? launch<2> : launch<4>)));
+  return run(p, ne, coords, conn, u, state, alpha_n, out, code, first_failure, stream);
 }
 
 }  // namespace sbk

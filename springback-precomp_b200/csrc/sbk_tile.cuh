@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 
 #include "sbk_element_math.cuh"
+#include "sbk_smem.h"
 #include "sbk_tile.h"
 #include "sbk_tile_point.cuh"
 #include "sbk_tile_search.cuh"
@@ -754,16 +755,10 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSm)
 
 template <int NT>
 int launch_tile(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream) {
-  static size_t raised[64] = {};
-  const size_t smem = tile_smem(a.elements, p.nq);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || raised[dev] < smem) {
-    cudaError_t err = cudaFuncSetAttribute(tile_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    if (dev >= 0 && dev < 64) raised[dev] = smem;
-  }
-  tile_kernel<NT><<<grid, kTileThreads, smem, stream>>>(p, a, s);
+  static SmemLimit limit;
+  const cudaError_t err = limit.allow(tile_kernel<NT>);
+  if (err != cudaSuccess) return (int)err;
+  tile_kernel<NT><<<grid, kTileThreads, tile_smem(a.elements, p.nq), stream>>>(p, a, s);
   return (int)cudaGetLastError();
 }
 
