@@ -845,7 +845,7 @@ struct Local {
       if (n <= kFullStepReduction * residual) break;
     }
     if (best_step == 0.0) return false;
-    if (!last_is_best) try_at(d, best_step);
+    if (!last_is_best && !try_at(d, best_step)) return false;
     advance(d, best_step);
     residual = best;
     return true;
@@ -893,7 +893,7 @@ struct Local {
     if (!evaluated) {
       if (s0 == 0.0) return false;
       step = s0;
-      try_at(d, step);
+      if (!try_at(d, step)) return false;
     }
     advance(d, step);
     residual = rnorm();

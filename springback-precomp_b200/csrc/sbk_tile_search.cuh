@@ -121,7 +121,10 @@ __device__ __noinline__ int search_after(E& e, TileSearch& s, bool evaluated, do
       return s.last_is_best ? 1 : search_trial(e, kStageBest, s.best_step);
     }
     default:  // kStageReturn, kStageBest
-      return 1;
+      // A point that evaluated before can fail now: its return starts from
+      // the closest point of the trial in between. The sums are then another
+      // trial's, so the element goes on as after any search that fails.
+      return evaluated ? 1 : 2;
   }
 }
 
