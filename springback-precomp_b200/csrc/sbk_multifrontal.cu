@@ -571,8 +571,6 @@ cudaError_t Multifrontal::build(const FrontOrder& order, const std::vector<int32
     child.insert(child.end(), fr.kids.begin(), fr.kids.end());
   }
   arena_ = (size_t)at;
-  const size_t bytes = (size_t)at * sizeof(double) + (size_t)diag_at * kPanel * kPanel * sizeof(double);
-  if (bytes > most) return cudaErrorMemoryAllocation;
   // A front's place of a row: its own columns first, then its rows below.
   auto place_in = [&](int f, int32_t row) {
     const int4& t = front[(size_t)f];
@@ -607,6 +605,31 @@ cudaError_t Multifrontal::build(const FrontOrder& order, const std::vector<int32
       }
   }
   entries_ = (int64_t)src.size();
+  // What the lists of tasks take is known before they are made: the tiles',
+  // one list a panel, grow with the cube of a front (a tenth of its own
+  // bytes at 40,000 rows).
+  int64_t num_adds = 0, num_panels = 0, num_tiles = 0;
+  for (int f = 0; f < nf; ++f) {
+    const int4& t = front[(size_t)f];
+    auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+    if (children[(size_t)f].y > 0) num_adds += up(t.z, kAddColumns);
+    for (int p0 = 0; p0 < t.y; p0 += kPanel) {
+      const int base = std::min(p0 + kPanel, t.y);
+      const int64_t tiles = up(t.z - base, kTile), own = up(t.y - base, kTile);
+      num_panels += std::max<int64_t>(1, up(t.z - base, kRowChunk));
+      num_tiles += own * (own + 1) / 2 + (tiles - own) * own;
+    }
+    const int64_t rest = up(t.z - t.y, kTile);
+    num_tiles += rest * (rest + 1) / 2;
+  }
+  auto some = [](int64_t n) { return (size_t)std::max<int64_t>(1, n); };  // as upload and room allocate
+  const size_t bytes =
+      (some(at) + some((int64_t)diag_at * kPanel * kPanel) + some(y_at)) * sizeof(double) +
+      some(nf) * (sizeof(int4) + sizeof(int2) + 2 * sizeof(int64_t) + 2 * sizeof(int32_t)) +
+      (some((int64_t)child.size()) + 2 * some((int64_t)rows.size()) + some(entries_)) * sizeof(int32_t) +
+      some(entries_) * sizeof(int64_t) + (some(num_adds) + some(num_panels)) * sizeof(int2) + some(num_tiles) * sizeof(int4);
+  if (bytes > most || std::max(num_tiles, std::max(num_panels, num_adds)) > INT32_MAX)
+    return cudaErrorMemoryAllocation;
   // Tasks, level by level.
   std::vector<int32_t> by_level;
   std::vector<int2> adds, panel_tasks;
@@ -695,7 +718,7 @@ cudaError_t Multifrontal::factor(const double* values, int32_t* failed, cudaStre
   const Fronts f{front_, offset_, arena_dev_};
   cudaError_t err = cudaMemsetAsync(arena_dev_, 0, arena_ * sizeof(double), stream);
   if (err != cudaSuccess) return err;
-  err = cudaMemsetAsync(failed, 0x7f, sizeof(int32_t), stream);
+  err = cudaMemsetAsync(failed, kAllPositive & 0xff, sizeof(int32_t), stream);
   if (err != cudaSuccess) return err;
   const int64_t blocks = std::min<int64_t>((entries_ + 255) / 256, 148 * 16);
   scatter_values_kernel<<<(unsigned)std::max<int64_t>(1, blocks), 256, 0, stream>>>(values, src_, dst_, entries_,

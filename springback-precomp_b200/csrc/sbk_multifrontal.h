@@ -37,11 +37,12 @@ class Multifrontal {
 
   // The fronts of the matrix whose CSR pattern (rowptr, col; in `order`) is
   // given, and their device storage. cudaErrorMemoryAllocation when that
-  // takes more than `most` bytes or is not to be had.
+  // takes more than `most` bytes, all tables counted, or is not to be had.
   cudaError_t build(const FrontOrder& order, const std::vector<int32_t>& rowptr, const std::vector<int32_t>& col,
                     size_t most);
-  // A = L L^T of the CSR values (device). *failed (device): a column of
-  // non-positive pivot, or 0x7fffffff.
+  // A = L L^T of the CSR values (device). *failed (device): the first column
+  // of non-positive pivot, or kAllPositive.
+  static constexpr int32_t kAllPositive = 0x7f7f7f7f;  // four bytes alike: a memset's
   cudaError_t factor(const double* values, int32_t* failed, cudaStream_t stream);
   // x = A^-1 b (device, in `order`; x and b may not alias).
   cudaError_t solve(const double* b, double* x, cudaStream_t stream);

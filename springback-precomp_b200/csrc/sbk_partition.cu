@@ -561,7 +561,7 @@ int chol_factor(sbk_partition* P, const double* values, bool* definite) {
     int32_t failed = 0;
     PCUDA(cudaMemcpyAsync(&failed, P->pivot, sizeof(failed), cudaMemcpyDeviceToHost, P->stream));
     PCUDA(cudaStreamSynchronize(P->stream));
-    *definite = failed == 0x7f7f7f7f;
+    *definite = failed == sbk::Multifrontal::kAllPositive;
     return SBK_OK;
   }
   PSOLVER(cusolverSpDcsrcholFactor(P->handle, P->nf, (int)P->nnz_ff, P->descr, values, P->fac_rowptr, P->fac_col,
