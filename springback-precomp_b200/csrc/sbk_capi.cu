@@ -466,6 +466,7 @@ int ensure_tile(sbk_system* s) {
   cudaError_t e = cudaMalloc(&s->tile_mem, sbk::tile_scratch_bytes(s->ne, s->p.nq));
   if (e != cudaSuccess) {
     s->tile_mem = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
     return fail(SBK_ERR_CUDA, std::string("cudaMalloc (tile scratch): ") + cudaGetErrorString(e));
   }
   sbk::tile_scratch_carve(s->tile_mem, s->ne, s->p.nq, s->tile);
@@ -699,12 +700,16 @@ int sbk_system_set_element(sbk_system* sys, int element, int mean_dilatation) {
     return fail(SBK_ERR_CONFIG,
                 "\"mean_dilatation\": \"all\" is not combined with the incompatible-mode Hex8: averaging the "
                 "dilatation of its modes leaves a zero-energy mode; use \"auto\" or \"none\"");
+  // The standard Hex8 has no kernel without the scratch: the element changes
+  // once it is there.
+  if (element == SBK_ELEMENT_STANDARD || sys->local_mode == SBK_LOCAL_PHASES)
+    if (int rc = ensure_tile(sys)) return rc;
   sys->p.element = element == SBK_ELEMENT_STANDARD ? 1 : 0;
   sys->p.averaged = (element == SBK_ELEMENT_STANDARD && mean_dilatation != SBK_MEAN_DILATATION_NONE && sys->p.nq > 1)
                         ? 1
                         : 0;
   sys->order_valid = false;
-  return sys->p.element == 1 || sys->local_mode == SBK_LOCAL_PHASES ? ensure_tile(sys) : SBK_OK;
+  return SBK_OK;
 }
 
 int sbk_system_set_frozen(sbk_system* sys, int frozen) {
