@@ -186,8 +186,10 @@ int sbk_system_set_elements_per_block(sbk_system* sys, int elements_per_block);
  * SBK_LOCAL_SINGLE_KERNEL: one kernel runs each element from start to
  * finish. The first keeps records of up to 1 GiB on the device (5.6 KB an
  * element at 8 points, 14.1 KB at 20; allocated by the system when it is
- * made or its element changes). sbk_set_local_iteration sets what sbk_element_batch
- * uses and what new systems start with. */
+ * made or its element changes), fewer where there is no memory for them:
+ * the elements then go in more launches, with the same results.
+ * sbk_set_local_iteration sets what sbk_element_batch uses and what new
+ * systems start with. */
 #define SBK_LOCAL_PHASES 0
 #define SBK_LOCAL_SINGLE_KERNEL 1
 int sbk_set_local_iteration(int mode);

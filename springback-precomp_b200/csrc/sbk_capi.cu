@@ -463,13 +463,9 @@ std::atomic<int> g_local_mode{SBK_LOCAL_PHASES};
 // capture).
 int ensure_tile(sbk_system* s) {
   if (s->tile_mem) return SBK_OK;
-  cudaError_t e = cudaMalloc(&s->tile_mem, sbk::tile_scratch_bytes(s->ne, s->p.nq));
-  if (e != cudaSuccess) {
-    s->tile_mem = nullptr;
-    cudaGetLastError();  // reported here, not by the next launch
-    return fail(SBK_ERR_CUDA, std::string("cudaMalloc (tile scratch): ") + cudaGetErrorString(e));
-  }
-  sbk::tile_scratch_carve(s->tile_mem, s->ne, s->p.nq, s->tile);
+  const cudaError_t e = sbk::tile_scratch_allocate(
+      s->ne, s->p.nq, [](void** p, size_t n) { return cudaMalloc(p, n); }, &s->tile_mem, s->tile);
+  if (e != cudaSuccess) return fail(SBK_ERR_CUDA, std::string("cudaMalloc (tile scratch): ") + cudaGetErrorString(e));
   return SBK_OK;
 }
 
@@ -561,9 +557,9 @@ int sbk_element_batch(const sbk_material* material, const sbk_rule* rule, int ki
   if (g_local_mode.load() == SBK_LOCAL_PHASES) {
     // The tile kernel's scratch, stream-ordered on the caller's stream.
     void* mem = nullptr;
-    SBK_CUDA(cudaMallocAsync(&mem, sbk::tile_scratch_bytes(ne, p.nq), s));
     sbk::TileScratch w;
-    sbk::tile_scratch_carve(mem, ne, p.nq, w);
+    SBK_CUDA(sbk::tile_scratch_allocate(
+        ne, p.nq, [s](void** at, size_t n) { return cudaMallocAsync(at, n, s); }, &mem, w));
     rc = sbk::launch_elements_tile(p, ne, x_dev, nullptr, u_dev, state_dev, alpha_dev, tangent_dev != nullptr,
                                    force_dev, tangent_dev, energy_dev, trial_dev, alpha_out_dev, yield_dev,
                                    iterations_dev, code_dev, nullptr, true, w, 0, s);

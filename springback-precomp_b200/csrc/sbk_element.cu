@@ -1613,24 +1613,11 @@ int launch_g(const Params& p, int64_t ne, const double* coords, const int32_t* c
 
 namespace {
 
-// Elements of a full tile: the points of a block's threads, at most
-// kTileMostElements.
-int tile_most(int nq) {
-  const int n = kTileThreads / nq;
-  return n < kTileMostElements ? n : kTileMostElements;
-}
-constexpr int kTileBlocks = 148 * kTileBlocksPerSm;  // resident at once
-
-}  // namespace
-
-namespace {
-
 // The arrays of a launch's scratch at base (NULL: their bytes only).
-size_t tile_layout(char* base, int64_t ne, int nq, TileScratch& s) {
+size_t tile_layout(char* base, int64_t ne, int nq, int64_t chunk, TileScratch& s) {
   const int most = tile_most(nq);
   const size_t points = (size_t)(most * nq) | 1;
   const size_t blocks = (size_t)(ne < kTileBlocks ? ne : kTileBlocks);
-  const size_t records = (size_t)(ne < tile_chunk(nq) ? ne : tile_chunk(nq));
   size_t at = 0;
   auto take = [&](size_t bytes) {
     char* here = base + at;
@@ -1640,24 +1627,25 @@ size_t tile_layout(char* base, int64_t ne, int nq, TileScratch& s) {
   s.counts = static_cast<int32_t*>(take(2 * sizeof(int32_t)));
   s.fallback = static_cast<int32_t*>(take((size_t)ne * sizeof(int32_t)));
   s.geo = static_cast<double*>(take(blocks * kTileGeo * points * sizeof(double)));
-  s.cond = static_cast<double*>(take(records * tile_record(nq) * sizeof(double)));
+  s.cond = static_cast<double*>(take((size_t)chunk * tile_record(nq) * sizeof(double)));
+  s.chunk = chunk;
   return at;
 }
 
 }  // namespace
 
-size_t tile_scratch_bytes(int64_t ne, int nq) {
+size_t tile_scratch_bytes(int64_t ne, int nq, int64_t chunk) {
   TileScratch s;
-  return tile_layout(nullptr, ne, nq, s);
+  return tile_layout(nullptr, ne, nq, chunk, s);
 }
 
-void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s) {
-  tile_layout(static_cast<char*>(base), ne, nq, s);
+void tile_scratch_carve(void* base, int64_t ne, int nq, int64_t chunk, TileScratch& s) {
+  tile_layout(static_cast<char*>(base), ne, nq, chunk, s);
 }
 
 namespace {
 
-// The element's kernels over the elements of `a`, in launches of tile_chunk, each
+// The element's kernels over the elements of `a`, in launches of s.chunk, each
 // followed by after(its arguments, its scratch).
 template <class After>
 int run_tiles(const Params& p, TileArgs a, const TileScratch& s, int elements_per_block, cudaStream_t stream,
@@ -1668,9 +1656,8 @@ int run_tiles(const Params& p, TileArgs a, const TileScratch& s, int elements_pe
   // tiles of 12, 327 us as 288 of 8; 8,192 of 8 points 190 and 178 us. From
   // five waves on there is no difference (23,086 of 8 points: 975 us).
   const int most = tile_most(p.nq);
-  const int64_t chunk = tile_chunk(p.nq);
-  for (a.begin = 0; a.begin < a.ne; a.begin += chunk) {
-    a.end = a.ne - a.begin < chunk ? a.ne : a.begin + chunk;
+  for (a.begin = 0; a.begin < a.ne; a.begin += s.chunk) {
+    a.end = a.ne - a.begin < s.chunk ? a.ne : a.begin + s.chunk;
     const int64_t n = a.end - a.begin, waves = (n + kTileBlocks * most - 1) / (kTileBlocks * most);
     a.elements = elements_per_block > 0 ? elements_per_block : (int)((n + kTileBlocks * waves - 1) / (kTileBlocks * waves));
     if (a.elements > most) a.elements = most;

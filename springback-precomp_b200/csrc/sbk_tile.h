@@ -23,7 +23,8 @@ struct TileScratch {
   int32_t* counts;    // [0] the next tile, [1] elements handed on
   int32_t* fallback;  // ne
   double* geo;        // blocks x kTileGeo x points of a tile
-  double* cond;       // tile_chunk x tile_record: the elements' records
+  double* cond;       // chunk x tile_record: the elements' records
+  int64_t chunk;      // elements of one launch
 };
 
 // Where an evaluation reads and writes (launch_elements' arguments).
@@ -79,9 +80,19 @@ __host__ __device__ inline size_t tile_record(int nq) {
   return cond_record(nq) > (size_t)kStdPoint * nq ? cond_record(nq) : (size_t)kStdPoint * nq;
 }
 
-// Elements of one launch: what 1 GiB of records holds (a mesh of more takes
-// several launches, so that the scratch does not grow with it).
-inline int64_t tile_chunk(int nq) { return (int64_t)((size_t(1) << 30) / (tile_record(nq) * sizeof(double))); }
+// Elements of a full tile: the points of a block's threads, at most
+// kTileMostElements.
+inline int tile_most(int nq) {
+  const int n = kTileThreads / nq;
+  return n < kTileMostElements ? n : kTileMostElements;
+}
+constexpr int kTileBlocks = 148 * kTileBlocksPerSm;  // resident at once
+
+// Elements of one launch: at most what 1 GiB of records holds (a mesh of more
+// takes several launches, so that the scratch does not grow with it), at
+// least, where there is no memory for that many, a wave of full tiles.
+inline int64_t tile_chunk_most(int nq) { return (int64_t)((size_t(1) << 30) / (tile_record(nq) * sizeof(double))); }
+inline int64_t tile_chunk_least(int nq) { return (int64_t)kTileBlocks * tile_most(nq); }
 
 // The condensation of the launch's elements whose code is 0: force and,
 // wanted, K*.
@@ -94,9 +105,28 @@ int launch_vjp_tile(const Params& p, const TileArgs& a, const TileScratch& s, co
 int launch_standard(const Params& p, const TileArgs& a, const TileScratch& s, cudaStream_t stream);
 
 // Bytes of one allocation that tile_scratch_carve splits, for ne elements of
-// nq points.
-size_t tile_scratch_bytes(int64_t ne, int nq);
-void tile_scratch_carve(void* base, int64_t ne, int nq, TileScratch& s);
+// nq points in launches of chunk.
+size_t tile_scratch_bytes(int64_t ne, int nq, int64_t chunk);
+void tile_scratch_carve(void* base, int64_t ne, int nq, int64_t chunk, TileScratch& s);
+
+// The scratch by allocate(void**, bytes), a smaller one where the device has
+// no memory for the full one: results do not depend on it, and a mesh that
+// fits the device is not refused for its scratch.
+template <class Allocate>
+cudaError_t tile_scratch_allocate(int64_t ne, int nq, Allocate allocate, void** mem, TileScratch& s) {
+  const int64_t least = tile_chunk_least(nq);
+  for (int64_t chunk = tile_chunk_most(nq) < ne ? tile_chunk_most(nq) : ne;; chunk /= 2) {
+    if (chunk < least) chunk = least < ne ? least : ne;
+    const cudaError_t err = allocate(mem, tile_scratch_bytes(ne, nq, chunk));
+    if (err == cudaSuccess) {
+      tile_scratch_carve(*mem, ne, nq, chunk, s);
+      return err;
+    }
+    *mem = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
+    if (err != cudaErrorMemoryAllocation || chunk <= least) return err;
+  }
+}
 
 // The tile kernel of the material's kind (one translation unit each).
 int launch_tile_j2(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);

@@ -1,6 +1,9 @@
-"""The tile kernels' scratch where device memory is short."""
+"""The tile kernels' scratch where device memory is short: a mesh whose own
+arrays fit is taken, its elements in more and smaller launches, with the
+same results to the bit."""
 from __future__ import annotations
 
+import contextlib
 import gc
 import importlib
 
@@ -27,9 +30,15 @@ def free_bytes():
     return torch.cuda.mem_get_info()[0]
 
 
-def leave(cuda, n):
-    """Takes the device's memory but n bytes."""
-    return torch.empty(max(0, free_bytes() - n), dtype=torch.uint8, device=cuda)
+@contextlib.contextmanager
+def only(cuda, n):
+    """Takes the device's memory but n bytes for a while."""
+    taken = [torch.empty(max(0, free_bytes() - n), dtype=torch.uint8, device=cuda)]
+    try:
+        yield
+    finally:
+        taken.clear()
+        free_bytes()
 
 
 def test_an_element_refused_for_memory_is_not_taken(pkg, cuda):
@@ -40,14 +49,59 @@ def test_an_element_refused_for_memory_is_not_taken(pkg, cuda):
     finally:
         system.set_local_iteration("phases")
     want = s.evaluate(u, 0.0, True).internal.cpu()
-    taken = leave(cuda, 8 * MB)
-    with pytest.raises(pkg.SbkError):
-        s.set_element("standard")
-    assert torch.equal(s.evaluate(u, 0.0, True).internal.cpu(), want)
-    s.commit()
-    del taken
-    free_bytes()
+    with only(cuda, 8 * MB):
+        with pytest.raises(pkg.SbkError):
+            s.set_element("standard")
+        assert torch.equal(s.evaluate(u, 0.0, True).internal.cpu(), want)
+        s.commit()
     s.set_element("standard")
     t, _ = sheet(pkg, cuda, "standard")
     t.set_committed(s.committed_all())
     assert torch.equal(s.evaluate(u, 0.0, True).internal.cpu(), t.evaluate(u, 0.0, True).internal.cpu())
+
+
+def results(s, u, standard):
+    ev = s.evaluate(u, 0.0, True)
+    out = [ev.internal.cpu(), ev.tangent.cpu(), torch.tensor([ev.energy, ev.gross, ev.yielding_points])]
+    out += [torch.tensor(s.trial_states()), torch.tensor(s.trial_modes())]
+    if not standard:
+        lam = torch.linspace(-1.0, 1.0, s.num_dofs, device=u.device, dtype=torch.float64)
+        out.append(s.vjp_x(u, lam, frozen=False).cpu())
+    return out
+
+
+@pytest.mark.parametrize("element", ["incompatible_modes", "standard"])
+def test_a_system_takes_smaller_launches(pkg, cuda, element):
+    s, u = sheet(pkg, cuda, element)
+    want = results(s, u, element == "standard")
+    assert 0 < want[2][2] < 20 * s.mesh.num_elements
+    before = free_bytes()
+    del s
+    whole = free_bytes() - before
+    assert whole > 300 * MB
+    with only(cuda, whole - 200 * MB):
+        s, _ = sheet(pkg, cuda, element)
+        got = results(s, u, element == "standard")
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_a_batch_takes_smaller_launches(pkg, cuda):
+    n, mat = 20000, pkg.material.hill_chaboche_sheet()
+    mesh = pkg.structured_hex_mesh(n, 1, 1, n * 1.0e-3, 1.0e-3, 1.0e-3)
+    x = torch.tensor(mesh.element_coordinates().reshape(n, 24), device=cuda)
+    gen = torch.Generator(device=cuda).manual_seed(6)
+    u = 4.0e-6 * torch.randn((n, 24), generator=gen, device=cuda, dtype=torch.float64)
+    state = torch.zeros((mat.state_fields, n, 20), device=cuda, dtype=torch.float64)
+
+    def run():
+        r = pkg.element_batch(mat, x, u, state, kinematics="logarithmic", thickness_points=5)
+        return [getattr(r, k).cpu() for k in ("force", "tangent", "energy", "states", "alpha", "code", "iterations")]
+
+    want = run()
+    assert (want[5] == 0).all() and (want[6] > 0).any()
+    outputs = sum(t.numel() * t.element_size() for t in want)
+    with only(cuda, outputs + 150 * MB):
+        got = run()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
