@@ -459,11 +459,30 @@ void free_system(sbk_system* s) {
 
 std::atomic<int> g_local_mode{SBK_LOCAL_PHASES};
 
+// The tile kernels' scratch by allocate(void**, bytes), a smaller one where the
+// device has no memory for the full one: results do not depend on it, and a
+// mesh that fits the device is not refused for its scratch.
+template <class Allocate>
+cudaError_t tile_scratch_allocate(int64_t ne, int nq, Allocate allocate, void** mem, sbk::TileScratch& s) {
+  const int64_t least = sbk::tile_chunk_least(nq);
+  for (int64_t chunk = sbk::tile_chunk_most(nq) < ne ? sbk::tile_chunk_most(nq) : ne;; chunk /= 2) {
+    if (chunk < least) chunk = least < ne ? least : ne;
+    const cudaError_t err = allocate(mem, sbk::tile_scratch_bytes(ne, nq, chunk));
+    if (err == cudaSuccess) {
+      sbk::tile_scratch_carve(*mem, ne, nq, chunk, s);
+      return err;
+    }
+    *mem = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
+    if (err != cudaErrorMemoryAllocation || chunk <= least) return err;
+  }
+}
+
 // The tile kernels' scratch of a system (allocated once, outside any stream
 // capture).
 int ensure_tile(sbk_system* s) {
   if (s->tile_mem) return SBK_OK;
-  const cudaError_t e = sbk::tile_scratch_allocate(
+  const cudaError_t e = tile_scratch_allocate(
       s->ne, s->p.nq, [](void** p, size_t n) { return cudaMalloc(p, n); }, &s->tile_mem, s->tile);
   if (e != cudaSuccess) return fail(SBK_ERR_CUDA, std::string("cudaMalloc (tile scratch): ") + cudaGetErrorString(e));
   return SBK_OK;
@@ -558,7 +577,7 @@ int sbk_element_batch(const sbk_material* material, const sbk_rule* rule, int ki
     // The tile kernel's scratch, stream-ordered on the caller's stream.
     void* mem = nullptr;
     sbk::TileScratch w;
-    SBK_CUDA(sbk::tile_scratch_allocate(
+    SBK_CUDA(tile_scratch_allocate(
         ne, p.nq, [s](void** at, size_t n) { return cudaMallocAsync(at, n, s); }, &mem, w));
     rc = sbk::launch_elements_tile(p, ne, x_dev, nullptr, u_dev, state_dev, alpha_dev, tangent_dev != nullptr,
                                    force_dev, tangent_dev, energy_dev, trial_dev, alpha_out_dev, yield_dev,

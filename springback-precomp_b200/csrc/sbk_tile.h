@@ -109,25 +109,6 @@ int launch_standard(const Params& p, const TileArgs& a, const TileScratch& s, cu
 size_t tile_scratch_bytes(int64_t ne, int nq, int64_t chunk);
 void tile_scratch_carve(void* base, int64_t ne, int nq, int64_t chunk, TileScratch& s);
 
-// The scratch by allocate(void**, bytes), a smaller one where the device has
-// no memory for the full one: results do not depend on it, and a mesh that
-// fits the device is not refused for its scratch.
-template <class Allocate>
-cudaError_t tile_scratch_allocate(int64_t ne, int nq, Allocate allocate, void** mem, TileScratch& s) {
-  const int64_t least = tile_chunk_least(nq);
-  for (int64_t chunk = tile_chunk_most(nq) < ne ? tile_chunk_most(nq) : ne;; chunk /= 2) {
-    if (chunk < least) chunk = least < ne ? least : ne;
-    const cudaError_t err = allocate(mem, tile_scratch_bytes(ne, nq, chunk));
-    if (err == cudaSuccess) {
-      tile_scratch_carve(*mem, ne, nq, chunk, s);
-      return err;
-    }
-    *mem = nullptr;
-    cudaGetLastError();  // reported here, not by the next launch
-    if (err != cudaErrorMemoryAllocation || chunk <= least) return err;
-  }
-}
-
 // The tile kernel of the material's kind (one translation unit each).
 int launch_tile_j2(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
 int launch_tile_general0(const Params& p, const TileArgs& a, const TileScratch& s, unsigned grid, cudaStream_t stream);
