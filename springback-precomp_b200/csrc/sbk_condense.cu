@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "sbk_element_math.cuh"
+#include "sbk_mma.cuh"
 #include "sbk_point_table.cuh"
 #include "sbk_smem.h"
 #include "sbk_tile.h"
@@ -32,14 +33,6 @@ constexpr int kKua = 0;    // 24 x 10: K_ua and f_u (over the record's points)
 constexpr int kC = 240;    // 9 x 25: K_au and r_a, then their solutions
 constexpr int kGeo = 8 * kTab;  // 8 x 11 behind the table
 constexpr int kExtra = 8 * kTab + 88;
-
-// d += a (8 x 4, row-major) b (4 x 8): lane l holds a[l / 4][l % 4],
-// b[l % 4][l / 4] and d[l / 4][2 (l % 4) + {0, 1}].
-__device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 // The record's points and, behind at least what K_ua and C take over them,
 // the element's own values; then the table.

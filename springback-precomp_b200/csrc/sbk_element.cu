@@ -143,12 +143,12 @@ __device__ __forceinline__ void vtensor(const double* slot, const double g[3], b
   }
 }
 
-// The per-element context of a group: S is the shared-memory record of one
+// The per-element context of a group: s is the shared-memory record of its
 // element.
-template <int G, class Rec = ElemShared<G>>
+template <int G>
 struct Ctx {
   const Params* p;
-  Rec* s;
+  ElemShared<G>* s;
   int lane;
   unsigned mask;
   int64_t e;
@@ -162,8 +162,8 @@ struct Ctx {
 };
 
 // Mode gradients of point q: g~(i, m) = (det0 / det)(-2 xi_m) J0^-1(m, i).
-template <int G, class Rec>
-__device__ __forceinline__ void mode_grads(const Ctx<G, Rec>& c, int q, double gt[9]) {
+template <int G>
+__device__ __forceinline__ void mode_grads(const Ctx<G>& c, int q, double gt[9]) {
   const double ratio = c.s->geo[q][10];
   const double nat[3] = {c.p->qp[q][0], c.p->qp[q][1], c.p->qp[q][2]};
 #pragma unroll
@@ -174,8 +174,8 @@ __device__ __forceinline__ void mode_grads(const Ctx<G, Rec>& c, int q, double g
   }
 }
 // Gradient of node a at point q: g(i) = sum_c dN_a/dxi_c J^-1(c, i).
-template <int G, class Rec>
-__device__ __forceinline__ void node_grad(const Ctx<G, Rec>& c, int q, int a, double g[3]) {
+template <int G>
+__device__ __forceinline__ void node_grad(const Ctx<G>& c, int q, int a, double g[3]) {
   double dn[3];
   shape_grad(a, c.p->qp[q][0], c.p->qp[q][1], c.p->qp[q][2], dn);
   const double* ji = c.s->geo[q];
@@ -185,9 +185,9 @@ __device__ __forceinline__ void node_grad(const Ctx<G, Rec>& c, int q, int a, do
 
 // Reference geometry (set_up, IncompatibleModes.cpp:134-192). Returns 0 or
 // SBK_EL_MESH_INVERTED (group-uniform).
-template <int G, class Rec>
-__device__ int set_up(const Ctx<G, Rec>& c) {
-  Rec& s = *c.s;
+template <int G>
+__device__ int set_up(const Ctx<G>& c) {
+  ElemShared<G>& s = *c.s;
   const Params& p = *c.p;
   // Centre Jacobian, every lane alike.
   double j0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -251,8 +251,8 @@ __device__ int set_up(const Ctx<G, Rec>& c) {
 // |H| entry, the strain the return takes and, under logarithmic
 // kinematics, the spectral data L of the log strain. Returns 0, or a
 // point-failure code (an inverted point, a log strain out of range).
-template <int G, class Rec>
-__device__ __forceinline__ int point_kinematics(const Ctx<G, Rec>& c, int q, const double at[9], double gt[9],
+template <int G>
+__device__ __forceinline__ int point_kinematics(const Ctx<G>& c, int q, const double at[9], double gt[9],
                                                 double F[9], double& hmax, double strain[6], LogKin& L) {
   const Params& p = *c.p;
   int code = 0;
@@ -306,17 +306,16 @@ __device__ __forceinline__ int point_kinematics(const Ctx<G, Rec>& c, int q, con
 
 // After the point's response r: its yield flag, the material block M and
 // stress S in the strain measure of the element (the logarithmic map, or
-// as they are), and its slot for the group sums. MAPPED: r already holds
-// them in the element's strain measure (the logarithmic map was applied).
-template <int G, class Rec, bool MAPPED = false>
-__device__ __forceinline__ void point_slot(const Ctx<G, Rec>& c, int q, const Response& r, const LogKin& L,
+// as they are), and its slot for the group sums.
+template <int G>
+__device__ __forceinline__ void point_slot(const Ctx<G>& c, int q, const Response& r, const LogKin& L,
                                            const double F[9], double w, double hmax, double M[36], double S[6]) {
   const Params& p = *c.p;
-  Rec& s = *c.s;
+  ElemShared<G>& s = *c.s;
   c.yield[c.e * p.nq + q] = r.yielding ? 1 : 0;
 #pragma unroll
   for (int i = 0; i < 36; ++i) M[i] = r.C[i];
-  if (!MAPPED && p.kinematics == SBK_FINITE_LOGARITHMIC) {
+  if (p.kinematics == SBK_FINITE_LOGARITHMIC) {
     log_transform(L, r.stress, S, M);
   } else {
 #pragma unroll
@@ -341,45 +340,10 @@ __device__ __forceinline__ void point_slot(const Ctx<G, Rec>& c, int q, const Re
 // the first failure in the reference's order (the earliest stage, then the
 // lowest point), else K_aa and the force, scale and floor sums. fail =
 // (stage << 8) | q of this lane's failure (0: none), code its code.
-// The nodal force f_u (24) and the energy of the pass from the points'
-// slots, in point order: lane a (a < 8) node a, lane 7 the energy.
-template <int G, class Rec>
-__device__ __forceinline__ void force_sums(const Ctx<G, Rec>& c) {
-  Rec& s = *c.s;
-  const Params& p = *c.p;
-  if (c.lane < 8) {
-    const int a = c.lane;
-    double ra[3] = {0, 0, 0}, en = 0.0;
-    for (int qq = 0; qq < p.nq; ++qq) {
-      const double* sl = s.slot[qq];
-      const double* Fq = sl + kSlotF;
-      const double* Sq = sl + kSlotS;
-      const double wq = sl[kSlotW];
-      double FS[9];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          FS[k * 3 + j] = Fq[k * 3 + 0] * Sq[voigt(0, j)] + Fq[k * 3 + 1] * Sq[voigt(1, j)] + Fq[k * 3 + 2] * Sq[voigt(2, j)];
-      double g[3];
-      node_grad(c, qq, a, g);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) ra[k] += wq * (FS[k * 3 + 0] * g[0] + FS[k * 3 + 1] * g[1] + FS[k * 3 + 2] * g[2]);
-      if (a == 7) en += wq * sl[kSlotE];
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s.r[3 * a + k] = ra[k];
-    if (a == 7) s.energy = en;
-  }
-  c.sync();
-}
-
-// FORCES = false leaves out the nodal force and the energy (force_sums
-// gives them, the same sums, for the pass that ends the iteration).
-template <int G, class Rec, bool FORCES = true>
-__device__ __forceinline__ int pass_sums(const Ctx<G, Rec>& c, bool active, int fail, int code, const double gt[9],
+template <int G>
+__device__ __forceinline__ int pass_sums(const Ctx<G>& c, bool active, int fail, int code, const double gt[9],
                                          const double F[9], const double M[36], const double S[6], double w) {
-  Rec& s = *c.s;
+  ElemShared<G>& s = *c.s;
   const Params& p = *c.p;
   const bool geometric = p.kinematics != SBK_SMALL_STRAIN;
   double kbuf[G];
@@ -476,12 +440,10 @@ __device__ __forceinline__ int pass_sums(const Ctx<G, Rec>& c, bool active, int 
 #pragma unroll
         for (int j = 0; j < 3; ++j)
           FS[k * 3 + j] = Fq[k * 3 + 0] * Sq[voigt(0, j)] + Fq[k * 3 + 1] * Sq[voigt(1, j)] + Fq[k * 3 + 2] * Sq[voigt(2, j)];
-      if (FORCES) {
-        double g[3];
-        node_grad(c, qq, a, g);
+      double g[3];
+      node_grad(c, qq, a, g);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) ra[k] += wq * (FS[k * 3 + 0] * g[0] + FS[k * 3 + 1] * g[1] + FS[k * 3 + 2] * g[2]);
-      }
+      for (int k = 0; k < 3; ++k) ra[k] += wq * (FS[k * 3 + 0] * g[0] + FS[k * 3 + 1] * g[1] + FS[k * 3 + 2] * g[2]);
       if (a < 3) {
         double gtq[9];
         mode_grads(c, qq, gtq);
@@ -501,11 +463,10 @@ __device__ __forceinline__ int pass_sums(const Ctx<G, Rec>& c, bool active, int 
           fl[k] += sl[kSlotFl] * s2;
         }
       }
-      if (FORCES && a == 7) en += wq * sl[kSlotE];
+      if (a == 7) en += wq * sl[kSlotE];
     }
-    if (FORCES)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) s.r[3 * a + k] = ra[k];
+    for (int k = 0; k < 3; ++k) s.r[3 * a + k] = ra[k];
     if (a < 3) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -514,18 +475,17 @@ __device__ __forceinline__ int pass_sums(const Ctx<G, Rec>& c, bool active, int 
         s.flo[3 * a + k] = fl[k];
       }
     }
-    if (FORCES && a == 7) s.energy = en;
+    if (a == 7) s.energy = en;
   }
   c.sync();
   return 0;
 }
 
-
 // One pass (IncompatibleModes.cpp:337-342): the kinematics, the returns and
 // the sums at `at` (9 values, identical in every lane). Returns 0 or the
 // failure code of the first failing point in the reference's order.
-template <int G, class Rec>
-__device__ __noinline__ int pass(const Ctx<G, Rec>& c, const double at[9]) {
+template <int G>
+__device__ __noinline__ int pass(const Ctx<G>& c, const double at[9]) {
   const Params& p = *c.p;
   const int q = c.lane;
   const bool active = q < p.nq;
@@ -564,9 +524,9 @@ __device__ __noinline__ int pass(const Ctx<G, Rec>& c, const double at[9]) {
 // scan takes it; rows, then columns exchanged; the column below the pivot
 // multiplied by its reciprocal, then the rank-one update. rowp / colp hold
 // the transpositions.
-template <int G, class CT>
-__device__ __forceinline__ bool fullpiv_lu9_rows_inline(const CT& c, const double* a, double* lu, int* rowp,
-                                                        int* colp, double* maxpivot_out) {
+template <int G>
+__device__ __noinline__ bool fullpiv_lu9_rows(const Ctx<G>& c, const double* a, double* lu, int* rowp, int* colp,
+                                              double* maxpivot_out) {
   const int lane = c.lane;
   _Pragma("unroll 1") for (int i = lane; i < 81; i += G) lu[i] = a[i];
   c.sync();
@@ -640,15 +600,9 @@ __device__ __forceinline__ bool fullpiv_lu9_rows_inline(const CT& c, const doubl
   return ok;
 }
 
-template <int G, class CT>
-__device__ __noinline__ bool fullpiv_lu9_rows(const CT& c, const double* a, double* lu, int* rowp, int* colp,
-                                              double* maxpivot_out) {
-  return fullpiv_lu9_rows_inline<G>(c, a, lu, rowp, colp, maxpivot_out);
-}
-
 // x = A^-1 b with the FullPivLU factors (any lane; b and x may alias).
-__device__ __forceinline__ void fullpiv_solve9_inline(const double* lu, const int* rowp, const int* colp,
-                                                      const double* b, double* x) {
+__device__ __noinline__ void fullpiv_solve9(const double* lu, const int* rowp, const int* colp, const double* b,
+                                            double* x) {
   double y[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) y[i] = b[i];
@@ -688,11 +642,6 @@ __device__ __forceinline__ void fullpiv_solve9_inline(const double* lu, const in
   }
 #pragma unroll
   for (int i = 0; i < 9; ++i) x[i] = y[i];
-}
-
-__device__ __noinline__ void fullpiv_solve9(const double* lu, const int* rowp, const int* colp, const double* b,
-                                            double* x) {
-  fullpiv_solve9_inline(lu, rowp, colp, b, x);
 }
 
 // x = A^-T b with the FullPivLU factors of A (P A Q = L U, so
@@ -745,8 +694,8 @@ __device__ __noinline__ void fullpiv_solve9_t(const double* lu, const int* rowp,
 // diagonal by the lane of row k, then the rows below in parallel, each entry
 // the same dot product in the same order - the same factor and the same
 // answer.
-template <int G, class CT>
-__device__ __forceinline__ bool llt9_rows_inline(const CT& c, double* a) {
+template <int G>
+__device__ __noinline__ bool llt9_rows(const Ctx<G>& c, double* a) {
   const int lane = c.lane;
   _Pragma("unroll 1") for (int k = 0; k < 9; ++k) {
     int bad = 0;
@@ -770,11 +719,6 @@ __device__ __forceinline__ bool llt9_rows_inline(const CT& c, double* a) {
     c.sync();
   }
   return true;
-}
-
-template <int G, class CT>
-__device__ __noinline__ bool llt9_rows(const CT& c, double* a) {
-  return llt9_rows_inline<G>(c, a);
 }
 
 // ---- the local iteration -------------------------------------------------------
@@ -1032,13 +976,11 @@ struct Local {
 // the tangent, K* = K_uu - K_ua C, symmetrised for a symmetric tangent. Reads
 // the group's shared record: the last pass's slots and sums (slot, r), the
 // factors of its K_aa (lu, rowp, colp) and the geometry; kc is overwritten.
-// INLINE_SOLVE: the 9 x 9 solves compiled in place (their vectors stay in
-// registers) rather than called.
-template <int G, class Rec, bool INLINE_SOLVE = false>
-__device__ __forceinline__ void condense(const Ctx<G, Rec>& c, int want_tangent, double* __restrict__ force,
+template <int G>
+__device__ __forceinline__ void condense(const Ctx<G>& c, int want_tangent, double* __restrict__ force,
                                          double* __restrict__ tangent) {
   const Params& p = *c.p;
-  Rec& s = *c.s;
+  ElemShared<G>& s = *c.s;
   const int lane = c.lane;
   const int64_t e = c.e;
   const bool sym = p.symmetric != 0;
@@ -1086,8 +1028,7 @@ __device__ __forceinline__ void condense(const Ctx<G, Rec>& c, int want_tangent,
 #pragma unroll
       for (int j = 0; j < 9; ++j) b[j] = sym ? kua[k][j] : kau[k][j];
       double x[9];
-      if (INLINE_SOLVE) fullpiv_solve9_inline(s.lu, s.rowp, s.colp, b, x);
-      else fullpiv_solve9(s.lu, s.rowp, s.colp, b, x);
+      fullpiv_solve9(s.lu, s.rowp, s.colp, b, x);
 #pragma unroll
       for (int j = 0; j < 9; ++j) C[(3 * a + k) * 9 + j] = x[j];
     }
@@ -1097,8 +1038,7 @@ __device__ __forceinline__ void condense(const Ctx<G, Rec>& c, int want_tangent,
     const int a = lane;
     // f* = f_u - K_ua K_aa^-1 r_alpha.
     double corr[9];
-    if (INLINE_SOLVE) fullpiv_solve9_inline(s.lu, s.rowp, s.colp, s.r + 24, corr);
-    else fullpiv_solve9(s.lu, s.rowp, s.colp, s.r + 24, corr);
+    fullpiv_solve9(s.lu, s.rowp, s.colp, s.r + 24, corr);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       double v = 0.0;
@@ -1731,10 +1671,6 @@ int launch_vjp(const Params& p, int64_t ne, const double* coords, const int32_t*
                     alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
   return run_list(vjp_kernel<32>, ne, 32, sizeof(ElemShared<32>), limit[1], stream, p, ne, coords, conn, u, state,
                   alpha_n, lambda, trial, yield, code, first_failure, out, s.fallback, s.counts + 1);
-}
-
-size_t element_smem_bytes(int group) {
-  return group == 8 ? sizeof(ElemShared<8>) : sizeof(ElemShared<32>);
 }
 
 int launch_elements(const Params& p, int64_t ne, const double* coords, const int32_t* conn, const double* u,

@@ -26,7 +26,6 @@ int launch_elements(const Params& p, int64_t ne, const double* coords, const int
                     double* energy, double* trial, double* alpha_out, uint8_t* yield, int32_t* iterations,
                     int32_t* code, int32_t* first_failure, bool batch, int elements_per_block,
                     const int32_t* order, cudaStream_t stream);
-size_t element_smem_bytes(int group);
 
 // K1 by tiles (sbk_tile.cuh; mesh or batch mode, as launch_elements), every
 // rule, and the standard Hex8 (sbk_standard.cu; mesh mode); no host

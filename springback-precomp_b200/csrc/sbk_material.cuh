@@ -19,14 +19,6 @@ namespace sbk {
 
 constexpr double kEps = 2.220446049250313e-16;
 
-// How the closest-point return's helpers (the residual evaluation, the
-// consistent tangent, the backstress decay) are compiled: as calls (one
-// copy of their code for every caller) unless a translation unit asks for
-// them inlined.
-#ifndef SBK_RETURN_HELPER
-#define SBK_RETURN_HELPER __noinline__
-#endif
-
 // Point-failure codes (sbk_element_code).
 constexpr int kFailInverted = SBK_EL_INVERTED_POINT;
 constexpr int kFailReturn = SBK_EL_RETURN_NO_CONVERGE;
@@ -219,7 +211,7 @@ __device__ __forceinline__ int radial_return(const Params& p, const double strai
 struct Decay {
   double theta, chi, dtheta, dchi;
 };
-static __device__ SBK_RETURN_HELPER Decay decay_of(double gamma, double dl, int integration) {
+static __device__ __noinline__ Decay decay_of(double gamma, double dl, int integration) {
   Decay d{1.0, 0.0, 0.0, 1.0};
   if (gamma == 0.0) {
     d.chi = dl;
@@ -253,7 +245,7 @@ struct Terms {
   double a[SBK_MAX_BACKSTRESSES][6];
 };
 
-static __device__ SBK_RETURN_HELPER bool gr_evaluate(const Params& p, const double s_trial[6], const Terms& tn,
+static __device__ __noinline__ bool gr_evaluate(const Params& p, const double s_trial[6], const Terms& tn,
                                             double a_n, const double xi[6], double dl, GPoint& e) {
   double pxi[6];
 #pragma unroll
@@ -390,7 +382,7 @@ __device__ __forceinline__ void j_solve(const Params& p, const GPoint& e, const 
 
 // C_alg = C^e - 2G [m_t a^T + (dl / sigma_bar) S (P - m m^T) A] with
 // [A; a^T] = J^-1 [D_dev; 0] (Plasticity.cpp:299-311).
-static __device__ SBK_RETURN_HELPER void gr_tangent(const Params& p, const GPoint& e, double a_n, double dl, double C[36]) {
+static __device__ __noinline__ void gr_tangent(const Params& p, const GPoint& e, double a_n, double dl, double C[36]) {
   JFactor jf;
   j_factor(p, e, a_n, dl, jf);
   const double g = p.G;
@@ -856,29 +848,6 @@ __device__ __forceinline__ double rot_m(const double q[9], int r, int c) {
   const int kc[6] = {0, 1, 2, 1, 2, 0};
   const int a = kr[r], b = kc[r], i = kr[c], j = kc[c];
   return i == j ? q[i * 3 + a] * q[i * 3 + b] : q[i * 3 + a] * q[j * 3 + b] + q[j * 3 + a] * q[i * 3 + b];
-}
-
-// S = P^T T alone (LogarithmicStrain.cpp:144-149): the second
-// Piola-Kirchhoff stress of the Kirchhoff-like stress T work-conjugate to
-// E_log, for stress recovery.
-static __device__ __noinline__ void log_stress(const LogKin& L, const double t[6], double s_out[6]) {
-  const int kr[6] = {0, 1, 2, 0, 1, 2};
-  const int kc[6] = {0, 1, 2, 1, 2, 0};
-  double tpv[6];
-#pragma unroll
-  for (int r = 0; r < 6; ++r) {
-    double v = 0.0;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) v += rot_m(L.q, r, c) * t[c];
-    tpv[r] = v;
-  }
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double v = 0.0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) v += rot_m(L.q, k, i) * ((k < 3 ? 1.0 : 2.0) * first_of(L.first, kr[k], kc[k])) * tpv[k];
-    s_out[i] = i < 3 ? v : 0.5 * v;
-  }
 }
 
 // S = P^T T, and material = P^T C P + T : L in global axes (engineering

@@ -28,6 +28,8 @@
 #include <algorithm>
 #include <numeric>
 
+#include "sbk_mma.cuh"
+
 namespace sbk {
 namespace {
 
@@ -156,12 +158,6 @@ __global__ void __launch_bounds__(kRowChunk)
 #pragma unroll
   for (int j = 0; j < kPanel; ++j)
     if (j < nb) A[(int64_t)(p0 + j) * m + row] = x[j];
-}
-
-__device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
 }
 
 // C -= P_i P_j^T of one 64 x 64 tile of the lower matrix below the columns P:

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "sbk_element.h"
+#include "sbk_mma.cuh"
 #include "sbk_point_table.cuh"
 #include "sbk_smem.h"
 #include "sbk_tile_point.cuh"
@@ -47,7 +48,7 @@ __device__ __forceinline__ void load_spectral(const PointRecord& r, LogKin& L) {
 }
 
 // P^T t: the second Piola-Kirchhoff stress of a stress work-conjugate to the
-// log strain (log_stress).
+// log strain (LogarithmicStrain.cpp:144-149).
 __device__ __forceinline__ void pull_back(const LogKin& L, const double t[6], double out[6]) {
   double tp[6];
   rotate_in(L.q, t, tp);
@@ -288,12 +289,6 @@ constexpr int kWarps = 4;
 // F, three zeros.
 constexpr int kTabF = 40, kTabZero = 55, kTab = 58;
 constexpr int kExtra = 8 * kTab + 64;
-
-__device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 __host__ __device__ inline int warp_doubles(int nq) {
   return (kStdPoint * nq > 576 ? kStdPoint * nq : 576) + kExtra;
