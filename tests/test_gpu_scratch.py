@@ -7,8 +7,11 @@ import contextlib
 import gc
 import importlib
 
+import numpy as np
 import pytest
 import torch
+
+from conftest import X_DISTORTED, deformation, oracle_to_device
 
 pytestmark = pytest.mark.gpu
 MB = 1 << 20
@@ -105,3 +108,37 @@ def test_a_batch_takes_smaller_launches(pkg, cuda):
         got = run()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["chaboche_steel", "perfectly_plastic"])
+def test_elements_handed_on_in_every_launch(pkg, orc, cuda, name):
+    """The list of the elements handed to the single kernel runs on over the
+    launches: reversals that search and that turn K_aa indefinite and elements
+    that fail, spread over all of them."""
+    n, mat = 20000, getattr(pkg.material, name)()
+    kw = dict(kinematics="logarithmic", in_plane=2, thickness=5)
+    X = X_DISTORTED.reshape(1, 24)
+    first = orc.elements(mat.as_dict(), X, deformation(X_DISTORTED, 0.02).reshape(1, 24), want_tangent=False, **kw)
+    kinds = np.stack([deformation(X_DISTORTED, 0.02 * f) for f in (-6.0, -10.0, -15.0, 1.3, 1.0)])
+    kinds[4, 10] = np.nan
+    m = len(kinds)
+    states, alpha = np.repeat(first["states"], m, axis=0), np.repeat(first["alpha"].reshape(1, 9), m, axis=0)
+    ref = orc.elements(mat.as_dict(), np.repeat(X, m, axis=0), kinds, states, alpha, **kw)
+    at = np.random.default_rng(8).integers(0, m, n)
+    dev = np.ascontiguousarray(oracle_to_device(states, mat.kinematic_terms)[:, at])
+    args = [torch.tensor(v, device=cuda) for v in (np.repeat(X, n, axis=0), kinds[at], dev, alpha[at])]
+
+    def run():
+        r = pkg.element_batch(mat, *args, kinematics="logarithmic", thickness_points=5)
+        return [getattr(r, k).cpu() for k in ("force", "tangent", "energy", "alpha", "code", "iterations", "states")]
+
+    want = run()
+    np.testing.assert_array_equal(want[4].numpy(), ref["status"][at])
+    outputs = sum(t.numel() * t.element_size() for t in want)
+    with only(cuda, outputs + 150 * MB):
+        got = run()
+    assert torch.equal(got[4], want[4])
+    ok = want[4] == 0
+    for a, b in zip(got[:6], want[:6]):
+        assert torch.equal(a[ok], b[ok])
+    assert torch.equal(got[6][:, ok], want[6][:, ok])
