@@ -83,8 +83,11 @@ class PartBatch:
         8-lane group per element, a point per lane, start to finish), each at
         a block shape - with CUDA events
         on the system's stream after one warm-up; keep the fastest and
-        return {candidate: ms}. No result depends on the choice. A bare
-        integer candidate is an elements-per-block of the current mode."""
+        return {candidate: ms}. No decision of the local iteration depends on
+        the choice, and no value does between block shapes; between the two
+        kernels the values differ in their last bits, so where two runs have to
+        agree to the bit, set the mode instead. A bare integer candidate is an
+        elements-per-block of the current mode."""
         self.system.set_timing(True)
         times = {}
         for cand in candidates:

@@ -304,9 +304,9 @@ class NonlinearSystem:
     def set_local_iteration(self, mode: str = "phases"):
         """How the incompatible-mode Hex8's local iteration runs: "phases"
         (the default: tiles of elements through the iteration's phases
-        together) or
-        "single" (one kernel per element from start to finish). No result
-        depends on it."""
+        together) or "single" (one kernel per element from start to finish).
+        No decision depends on it - yield flags, iteration counts and failure
+        codes are the same - and the values only in their last bits."""
         _capi.check(_capi.lib().sbk_system_set_local_iteration(self._h, LOCAL_ITERATION[mode]))
 
     def set_values_buffer(self, values: Optional[torch.Tensor] = None):
