@@ -205,6 +205,8 @@ extern "C" int sbk_evaluate_noalloc(const sbk_material* material, const sbk_rule
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t err = cudaMemsetAsync(&s->first_failure, 0x7f, sizeof(int32_t), st);
   if (err != cudaSuccess) return sbk::set_error(SBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(err));
+  // The single kernel, which keeps nothing between kernels: the tiles' records
+  // would take 11 MB more of every GPU at 8 points, 29 MB at 20.
   rc = sbk::launch_elements(p, num_elements, coords_dev, connectivity_dev, u_dev, state_dev, alpha_dev,
                             values_dev != nullptr, s->force, s->tangent, s->energy, trial_dev, alpha_out_dev,
                             yield_dev, s->iterations, s->code, &s->first_failure, false, 0, nullptr, st);
