@@ -22,7 +22,8 @@
 // the chain of levels and panels, some hundred launches of a few microseconds
 // for a sheet of 13,689 rows. Measured there (41 x 41 x 3 nodes, clamped):
 // factorisation and one solve 44.7 ms with the level-scheduled sparse Cholesky
-// of the library, 1.5 ms so.
+// of the library, 1.5 ms so (2.0 ms with the refinement a symmetric solve takes,
+// sbk_partition.cu).
 #include "sbk_multifrontal.h"
 
 #include <algorithm>
